@@ -499,6 +499,7 @@ struct __align__(16) WarpSmem {
   float buf[kRowFloats];
   ListSmem list;
   NBatch nb;
+  FeeState fee;
 };
 template <>
 struct __align__(16) WarpSmem<true> {
@@ -647,14 +648,15 @@ __global__ void __launch_bounds__(kAccWarps * kWarp, 5) k_lut_pixels(AccumArgs a
       continue;
     }
     float loss = 0.f;
+    RowStats rs{0.f, 0.f, false};
     if constexpr (!VJP) {
       // ---- front end on the output ticks (row + 1)
       const float *nrm = a.normals ? a.normals + (int64_t)r * (1 + 3 * H) : nullptr;
       float *adc_dst = a.adc_out ? a.adc_out + (int64_t)r * H : nullptr;
       float *tick_dst = a.tick_out ? a.tick_out + (int64_t)r * H : nullptr;
-      warp_cumsum_charge(row + 1, T, p.t_sampling, lane);
+      rs = warp_cumsum_charge(row + 1, T, p.t_sampling, lane);
       if (MODE == kModeAdc) {
-        fee_forward(p, row + 1, T, nrm, adc_dst, tick_dst, nullptr, nullptr, early_exit, lane);
+        fee_forward(p, row + 1, T, rs, nrm, adc_dst, tick_dst, &sm.fee, false, nullptr, early_exit, lane);
         continue;
       }
     }
@@ -662,7 +664,8 @@ __global__ void __launch_bounds__(kAccWarps * kWarp, 5) k_lut_pixels(AccumArgs a
       const float *nrm = a.normals ? a.normals + (int64_t)r * (1 + 3 * H) : nullptr;
       float *adc_dst = a.adc_out ? a.adc_out + (int64_t)r * H : nullptr;
       float *tick_dst = a.tick_out ? a.tick_out + (int64_t)r * H : nullptr;
-      fee_forward(p, row + 1, T, nrm, adc_dst, tick_dst, &sm.fee, nullptr, early_exit, lane);
+      const bool swept =
+          fee_forward(p, row + 1, T, rs, nrm, adc_dst, tick_dst, &sm.fee, true, nullptr, early_exit, lane);
       // loss terms and digitisation adjoint, lane h for hit h
       if (lane < H) {
         const float raw = sm.fee.raw[lane];
@@ -679,7 +682,7 @@ __global__ void __launch_bounds__(kAccWarps * kWarp, 5) k_lut_pixels(AccumArgs a
       }
       loss = warp_sum(loss);
       __syncwarp();
-      fee_backward(p, row + 1, T, &sm.fee, sm.gint, lane);
+      fee_backward(p, row + 1, T, &sm.fee, sm.gint, swept, lane);
       if (lane == 0) row[0] = 0.f;
       __syncwarp();
     }

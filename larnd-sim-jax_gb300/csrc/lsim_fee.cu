@@ -21,10 +21,11 @@ constexpr int kFeeRow = 2048;
 
 // ---------------------------------------------------------------- FEE on wfs
 
-__global__ void __launch_bounds__(kFeeWarps * kWarp)
+__global__ void __launch_bounds__(kFeeWarps * kWarp, 6)
     k_fee(LsimParams p, const float *__restrict__ wfs, int64_t n_pix, int32_t T, const float *__restrict__ normals,
           float *adc_out, float *tick_out, float *integral_out) {
   __shared__ __align__(16) float rows[kFeeWarps][kFeeRow];
+  __shared__ FeeState fs[kFeeWarps];
   const int lane = threadIdx.x % kWarp, wid = threadIdx.x / kWarp;
   float *C = rows[wid];
   const int H = p.max_adc_values;
@@ -38,9 +39,9 @@ __global__ void __launch_bounds__(kFeeWarps * kWarp)
       for (int i = lane; i < T; i += kWarp) C[i] = __ldg(src + i);
     }
     __syncwarp();
-    warp_cumsum_charge(C, T, p.t_sampling, lane);
+    const RowStats rs = warp_cumsum_charge(C, T, p.t_sampling, lane);
     const float *nrm = normals ? normals + r * (1 + 3 * H) : nullptr;
-    fee_forward(p, C, T, nrm, adc_out + r * H, tick_out + r * H, nullptr,
+    fee_forward(p, C, T, rs, nrm, adc_out + r * H, tick_out + r * H, &fs[wid], false,
                 integral_out ? integral_out + r * H : nullptr, normals == nullptr && p.threshold > 0.f, lane);
     __syncwarp();
   }
@@ -62,7 +63,7 @@ int run_fee(const LsimParams &p, const float *wfs, int64_t n_pix, int32_t n_t, c
 // dL/dwfs of the front end + digitize for a cotangent on the ADCs: the
 // forward is recomputed per row (reset masks kept per warp in the
 // workspace), then the same adjoint the fused LUT gradient runs.
-__global__ void __launch_bounds__(kFeeWarps * kWarp)
+__global__ void __launch_bounds__(kFeeWarps * kWarp, 6)
     k_fee_vjp(LsimParams p, const float *__restrict__ wfs, int64_t n_pix, int32_t T, const float *__restrict__ normals,
               const float *__restrict__ g_adc, float *__restrict__ g_wfs, uint32_t *masks) {
   __shared__ __align__(16) float rows[kFeeWarps][kFeeRow];
@@ -80,13 +81,13 @@ __global__ void __launch_bounds__(kFeeWarps * kWarp)
     float4 *c4 = reinterpret_cast<float4 *>(C);
     for (int i = lane; i < T / 4; i += kWarp) c4[i] = __ldg(s4 + i);
     __syncwarp();
-    warp_cumsum_charge(C, T, p.t_sampling, lane);
+    const RowStats rs = warp_cumsum_charge(C, T, p.t_sampling, lane);
     const float *nrm = normals ? normals + r * (1 + 3 * H) : nullptr;
-    fee_forward(p, C, T, nrm, nullptr, nullptr, &st, nullptr, early_exit, lane);
+    const bool swept = fee_forward(p, C, T, rs, nrm, nullptr, nullptr, &st, true, nullptr, early_exit, lane);
     __syncwarp();
     if (lane < H) gint[wid][lane] = digitize_vjp(p, st.raw[lane], g_adc[r * H + lane]);
     __syncwarp();
-    fee_backward(p, C, T, &st, gint[wid], lane);
+    fee_backward(p, C, T, &st, gint[wid], swept, lane);
     float4 *d4 = reinterpret_cast<float4 *>(g_wfs + r * (int64_t)T);
     for (int i = lane; i < T / 4; i += kWarp) d4[i] = c4[i];
     __syncwarp();
