@@ -674,7 +674,7 @@ int lsim_param_stage2(const LsimParams *p, const void *ws, int64_t n_rows, int32
   AccumArgs a = make_args(p, nullptr, ws, n_rows, n_events);
   rc = run_fill_unique(*p, a.w, a.g, p_pad, n_em1, n_valid, unique_pixels, wfs, p->n_ticks - 1, st);
   if (rc) return wrap(rc, "lsim_param_stage2");
-  return wrap(run_param_accum(*p, a.w, a.g, n_valid, p_pad - n_valid, wfs, st), "lsim_param_stage2");
+  return wrap(run_param_accum(*p, a.w, a.g, n_valid, p_pad - n_valid, wfs, n_rows, st), "lsim_param_stage2");
 }
 
 int lsim_param_wfs_vjp(const LsimParams *p, const void *ws, int64_t n_rows, int32_t n_events, const float *g_wfs,

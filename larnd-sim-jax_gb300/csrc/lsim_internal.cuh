@@ -43,7 +43,7 @@ int run_main_records(const AccumArgs &a, cudaStream_t st);
 int run_main_adjoint(const AccumArgs &a, cudaStream_t st);
 
 int run_param_accum(const LsimParams &p, const Workspace &w, const Grid &g, int32_t n_valid, int64_t row_offset,
-                    float *wfs, cudaStream_t st);
+                    float *wfs, int64_t n_rows, cudaStream_t st);
 
 // lsim_fee.cu
 int run_fee(const LsimParams &p, const float *wfs, int64_t n_pix, int32_t n_t, const float *normals, float *adc_out,
