@@ -444,7 +444,9 @@ int lsim_chop_tracks(const LsimFieldMap *f, const float *tracks, int64_t n_rows,
 int lsim_pixel_coords(const LsimParams *p, const int32_t *unique_pixels, int64_t n_pix, float *x_out, float *y_out,
                       int32_t *plane_out, int32_t *event_out, void *stream);
 
-/* Workspace bytes of lsim_fee_prob (one flag per hit step). */
+/* Workspace bytes of lsim_fee_prob on the current device, for any number of
+ * pixels and paths (one flag per hit step, and the kernel blocks' scratch for
+ * path values: about 240 MB at 152 SMs). */
 size_t lsim_fee_prob_workspace_bytes(const LsimParams *p);
 
 /* Probabilistic self-trigger front end on waveforms wfs[n_pix][n_t]
@@ -462,7 +464,26 @@ int lsim_fee_prob(const LsimParams *p, const float *wfs, int64_t n_pix, int32_t 
                   float stop_threshold, float *log_prob_out, float *charge_out, float *exp_tick_out,
                   float *exp_adc_out, float *lambda_out, void *ws, size_t ws_bytes, void *stream);
 
-/* Workspace bytes of lsim_fee_prob_vjp (the forward's per-step path states). */
+/* Bytes of the record of a forward that lsim_fee_prob_vjp_recorded reads. */
+size_t lsim_fee_prob_record_bytes(const LsimParams *p, int64_t n_pix, int32_t n_paths);
+
+/* lsim_fee_prob that also writes the adjoint's record (each step's paths,
+ * selected ticks and ticks with a probability) to record. */
+int lsim_fee_prob_record(const LsimParams *p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
+                         float stop_threshold, float *log_prob_out, float *charge_out, float *exp_tick_out,
+                         float *exp_adc_out, float *lambda_out, void *record, size_t record_bytes, void *ws,
+                         size_t ws_bytes, void *stream);
+
+/* Vector-Jacobian product as lsim_fee_prob_vjp, on the record of a forward on
+ * the same waveforms instead of a re-run.  A cotangent on the
+ * log-probabilities or charges needs a record made with log_prob_out or
+ * charge_out. */
+int lsim_fee_prob_vjp_recorded(const LsimParams *p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
+                               const void *record, size_t record_bytes, const float *g_log_prob,
+                               const float *g_charge, const float *g_e_tick, const float *g_e_adc,
+                               const float *g_lambda, float *g_wfs, void *stream);
+
+/* Workspace bytes of lsim_fee_prob_vjp (the forward's workspace and record). */
 size_t lsim_fee_prob_vjp_workspace_bytes(const LsimParams *p, int64_t n_pix, int32_t n_paths);
 
 /* Vector-Jacobian product of lsim_fee_prob with respect to the waveforms:

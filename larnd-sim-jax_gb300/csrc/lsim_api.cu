@@ -397,23 +397,73 @@ size_t lsim_fee_prob_workspace_bytes(const LsimParams *p) {
   return p ? fee_prob_workspace_bytes(p->max_adc_values) : 0;
 }
 
+static int fee_prob(const LsimParams *p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
+                    float stop_threshold, float *log_prob_out, float *charge_out, float *exp_tick_out,
+                    float *exp_adc_out, float *lambda_out, void *record, void *ws, size_t ws_bytes, void *stream,
+                    const char *name) {
+  if (n_pix < 0 || (n_pix > 0 && !wfs)) return fail(LSIM_ERR_INVALID, "%s: bad waveform arguments", name);
+  const bool any_red = exp_tick_out || exp_adc_out || lambda_out;
+  if (any_red && !(exp_tick_out && exp_adc_out && lambda_out))
+    return fail(LSIM_ERR_INVALID, "%s: give all three of exp_tick, exp_adc, lambda or none", name);
+  if (!(stop_threshold > 0.0f)) return fail(LSIM_ERR_INVALID, "%s: stop_threshold %g", name, stop_threshold);
+  if (!ws || ws_bytes < fee_prob_workspace_bytes(p->max_adc_values))
+    return fail(LSIM_ERR_CAPACITY, "%s: workspace %zu < %zu bytes", name, ws_bytes,
+                fee_prob_workspace_bytes(p->max_adc_values));
+  return wrap(run_fee_prob(*p, wfs, n_pix, n_t, n_paths, stop_threshold, log_prob_out, charge_out, exp_tick_out,
+                           exp_adc_out, lambda_out, record, ws, (cudaStream_t)stream),
+              name);
+}
+
 int lsim_fee_prob(const LsimParams *p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
                   float stop_threshold, float *log_prob_out, float *charge_out, float *exp_tick_out,
                   float *exp_adc_out, float *lambda_out, void *ws, size_t ws_bytes, void *stream) {
   g_err.clear();
-  int rc = check_params(p);
+  const int rc = check_params(p);
   if (rc) return rc;
-  if (n_pix < 0 || (n_pix > 0 && !wfs)) return fail(LSIM_ERR_INVALID, "lsim_fee_prob: bad waveform arguments");
-  const bool any_red = exp_tick_out || exp_adc_out || lambda_out;
-  if (any_red && !(exp_tick_out && exp_adc_out && lambda_out))
-    return fail(LSIM_ERR_INVALID, "lsim_fee_prob: give all three of exp_tick, exp_adc, lambda or none");
-  if (!(stop_threshold > 0.0f)) return fail(LSIM_ERR_INVALID, "lsim_fee_prob: stop_threshold %g", stop_threshold);
-  if (!ws || ws_bytes < fee_prob_workspace_bytes(p->max_adc_values))
-    return fail(LSIM_ERR_CAPACITY, "lsim_fee_prob: workspace %zu < %zu bytes", ws_bytes,
-                fee_prob_workspace_bytes(p->max_adc_values));
-  return wrap(run_fee_prob(*p, wfs, n_pix, n_t, n_paths, stop_threshold, log_prob_out, charge_out, exp_tick_out,
-                           exp_adc_out, lambda_out, ws, (cudaStream_t)stream),
-              "lsim_fee_prob");
+  return fee_prob(p, wfs, n_pix, n_t, n_paths, stop_threshold, log_prob_out, charge_out, exp_tick_out, exp_adc_out,
+                  lambda_out, nullptr, ws, ws_bytes, stream, "lsim_fee_prob");
+}
+
+size_t lsim_fee_prob_record_bytes(const LsimParams *p, int64_t n_pix, int32_t n_paths) {
+  return p && n_pix >= 0 && n_paths > 0 ? fee_prob_record_bytes(n_pix, p->max_adc_values, n_paths) : 0;
+}
+
+static int check_record(const LsimParams *p, int64_t n_pix, int32_t n_paths, const void *record, size_t bytes,
+                        const char *name) {
+  if (n_pix < 0) return fail(LSIM_ERR_INVALID, "%s: bad waveform arguments", name);
+  if (n_paths < 1 || n_paths > 32) return fail(LSIM_ERR_UNSUPPORTED, "%s: n_paths %d", name, n_paths);
+  const size_t need = fee_prob_record_bytes(n_pix, p->max_adc_values, n_paths);
+  if (!record || bytes < need) return fail(LSIM_ERR_CAPACITY, "%s: record %zu < %zu bytes", name, bytes, need);
+  return LSIM_OK;
+}
+
+int lsim_fee_prob_record(const LsimParams *p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
+                         float stop_threshold, float *log_prob_out, float *charge_out, float *exp_tick_out,
+                         float *exp_adc_out, float *lambda_out, void *record, size_t record_bytes, void *ws,
+                         size_t ws_bytes, void *stream) {
+  g_err.clear();
+  int rc = check_params(p);
+  if (!rc) rc = check_record(p, n_pix, n_paths, record, record_bytes, "lsim_fee_prob_record");
+  if (rc) return rc;
+  return fee_prob(p, wfs, n_pix, n_t, n_paths, stop_threshold, log_prob_out, charge_out, exp_tick_out, exp_adc_out,
+                  lambda_out, record, ws, ws_bytes, stream, "lsim_fee_prob_record");
+}
+
+int lsim_fee_prob_vjp_recorded(const LsimParams *p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
+                               const void *record, size_t record_bytes, const float *g_log_prob,
+                               const float *g_charge, const float *g_e_tick, const float *g_e_adc,
+                               const float *g_lambda, float *g_wfs, void *stream) {
+  g_err.clear();
+  int rc = check_params(p);
+  if (!rc) rc = check_record(p, n_pix, n_paths, record, record_bytes, "lsim_fee_prob_vjp_recorded");
+  if (rc) return rc;
+  if (n_pix > 0 && (!wfs || !g_wfs)) return fail(LSIM_ERR_INVALID, "lsim_fee_prob_vjp_recorded: null pointer");
+  const bool any_red = g_e_tick || g_e_adc || g_lambda;
+  if (any_red && !(g_e_tick && g_e_adc && g_lambda))
+    return fail(LSIM_ERR_INVALID, "lsim_fee_prob_vjp_recorded: give all three reduction cotangents or none");
+  return wrap(run_fee_prob_vjp_recorded(*p, wfs, n_pix, n_t, n_paths, record, g_log_prob, g_charge, g_e_tick,
+                                        g_e_adc, g_lambda, g_wfs, (cudaStream_t)stream),
+              "lsim_fee_prob_vjp_recorded");
 }
 
 size_t lsim_fee_prob_vjp_workspace_bytes(const LsimParams *p, int64_t n_pix, int32_t n_paths) {

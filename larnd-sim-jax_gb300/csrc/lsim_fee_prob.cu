@@ -3,18 +3,17 @@
 // its step _find_one_hit_step (:334-384) and log_diff_ndtr (:33-53), plus
 // the per-hit reductions of get_average_hit_values (:463-480).
 //
-// One 256-thread block per pixel (persistent over pixels).  The block keeps
+// One 512-thread block per pixel (persistent over pixels).  The block keeps
 // the pixel's cumulative charge q, its running maximum and its suffix
 // maximum in shared memory; because max(x - c) = max(x) - c holds exactly
 // in floating point, the per-path running maxima of q - c are read from the
 // two shared arrays instead of being rescanned for each of the K paths.
 // Ticks whose inputs are bit-identical to the previous tick's are grouped
 // into classes (one evaluation per class; flat stretches of a waveform
-// collapse).  For each of the H hit steps the block walks the K paths and
-// every thread folds its classes into three online log-sum-exp
-// accumulators (hit, total, selection), with no barrier between paths.  A
-// block top-K over the
-// selection values (largest first, lower tick first on ties, as lax.top_k)
+// collapse).  For each of the H hit steps the block evaluates the paths whose
+// charge is new and every thread folds its classes' values of the K paths
+// into three online log-sum-exp accumulators (hit, total, selection).  A
+// block top-K over the selection values (largest first, lower tick first on ties, as lax.top_k)
 // gives the next K paths.  The reference stops the whole batch once no pixel
 // keeps a total path probability above stop_threshold; the step kernel
 // records per step whether any pixel stayed active and a second kernel
@@ -126,22 +125,9 @@ __device__ __forceinline__ void lse_merge(float &m, float &s, float m2, float s2
   }
 }
 
-__device__ __forceinline__ bool better(float va, int ia, float vb, int ib) {
-  return va > vb || (va == vb && ia < ib);
-}
-
-// warp-wide best (value, index) under better(); every lane gets the result
-__device__ __forceinline__ void warp_best(float &bv, int &bi) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    if (better(ov, oi, bv, bi)) {
-      bv = ov;
-      bi = oi;
-    }
-  }
-}
+// floats (no NaN) as unsigned integers in the same order, 0 below them all
+__device__ __forceinline__ unsigned order_key(float x) { return (unsigned)float_key(x) ^ 0x80000000u; }
+__device__ __forceinline__ float key_order(unsigned k) { return key_float((int)(k ^ 0x80000000u)); }
 
 // ---------------------------------------------------------------- block scans over a pixel row
 
@@ -212,10 +198,28 @@ struct ProbArgs {
   int T, K, interval;
   float z, thr, log_stop;
   float *log_prob, *charge, *e_tick, *e_adc, *lam;
+  unsigned long long *work;   // pixels handed out beyond the blocks' first
   int32_t *step_active;   // [H]: some pixel kept a total path probability above the stop level after step h
-  float *state;           // optional [n_pix][H][2][K]: each step's input path charges and log-probabilities
-  int32_t *state_top;     // optional [n_pix][H][K]: each step's selected ticks (for the adjoint)
+  float *cache;           // [blocks][K][kCacheArrays][kProbMaxT]: path values kept from step to step
+  bool all_steps;         // run every step even when nothing can come of it
+  // record for the adjoint (all or none):
+  float *state;           // [n_pix][H][2][K]: each step's input path charges and log-probabilities
+  int32_t *state_top;     // [n_pix][H][K]: each step's selected ticks
+  uint32_t *live;         // [n_pix][H][kLiveWords]: ticks whose probability is not 0
+  int32_t *n_run;         // [n_pix]: steps run
+  float *red;             // [3][n_pix][H]: expected tick and ADC, total probability
 };
+
+constexpr int kCacheArrays = 3;               // per path: dist, selection and hit value of each class
+constexpr float kNoHit = 2.0f;                // a hit value (never above 0) that has not been formed yet
+constexpr int kLiveWords = kProbMaxT / 32;
+// exp of anything below is 0 in float32 (half of the smallest denormal is e^-103.97)
+constexpr float kProbDead = -104.0f;
+// a path's hit term below this leaves a log-sum-exp above kProbDead as it is:
+// 32 terms of e^-26 next to 1 are below its rounding
+constexpr float kProbFar = kProbDead - 26.0f;
+// log_diff_ndtr(a, b) <= -1000 sigmoid(-1000 (a - b)): below -1000 sigmoid(-1.4) = -197.8 for a - b < 1.4e-3
+constexpr float kWeakRise = 1.4f, kWeakMost = -190.0f;
 
 // The per-tick work of a step reads, for tick t, only the running maximum
 // at t and t+1, q at t, t+1, s = shifted(t) and s+1, and the suffix maximum
@@ -224,14 +228,40 @@ struct ProbArgs {
 // evaluates one representative per run of equal ticks (a "class") and
 // expands the class values back to ticks; flat stretches of a waveform
 // (no charge arriving) collapse to a handful of classes.
+//
+// What a path adds to a class depends on its charge alone (its probability
+// enters the log-sum-exps), and two thirds of a pixel's paths carry a charge
+// that a path of the step before carried (after the last real hit the top-K
+// ticks hardly change).  So the values of a path are kept in the block's
+// scratch (global memory, in L2) for as long as some path has its charge:
+// a step evaluates new charges only and then folds the K paths' kept values,
+// in the order and with the operations of an evaluation in place.
+//
+// Without the distributions (kDist false) a value matters only where its
+// probability does not underflow, and the rest is left out exactly:
+// * a tick on which the running maximum rises by less than kWeakRise / 1000
+//   noise widths has dist terms below kWeakMost for every path (the smooth
+//   gate's floor), so only the classes of the other ticks, 10 to 30 % of them,
+//   are evaluated; a path selected on such a tick could add nothing that
+//   float32 keeps.  Where fewer than K ticks are left, the paths that are
+//   missing repeat the best path's charge at the floor's probability, as the
+//   first step's do, and are skipped.  Should a tick with a likely dist value
+//   have to compete with the ticks left out (its own selection value is below
+//   theirs could be), the pixel starts over with all classes;
+// * hit <= dist, so the hit terms are formed only for the (class, path) pairs
+//   whose dist term is above kProbFar;
+// * a pixel whose paths have all become improbable beyond kProbDead stops.
+// Bound by instruction issue in the special functions.  Values and gradient of
+// 1500 dense rows: 42.4 -> 10.1 ms; distributions of 1000 rows: 8.8 -> 5.2 ms.
+template <bool kDist>
 __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob(ProbArgs a) {
   extern __shared__ __align__(16) float sm[];
   float *qs = sm, *cm = qs + kProbMaxT, *cr = cm + kProbMaxT, *esp = cr + kProbMaxT, *sw = esp + kProbMaxT;
   float *vh = sw + kProbMaxT, *vd = vh + kProbMaxT, *vs = vd + kProbMaxT;
   int *cls = reinterpret_cast<int *>(vs + kProbMaxT), *rep = cls + kProbMaxT;
   float *part = reinterpret_cast<float *>(rep + kProbMaxT);   // [kProbThreads][6] partial sums of path groups
-  float *cand_v = part + 6 * kProbThreads;                     // [warps][K] per-warp top-K candidates
-  int *cand_i = reinterpret_cast<int *>(cand_v + (kProbThreads / 32) * kProbMaxPaths);
+  unsigned *cand_k = reinterpret_cast<unsigned *>(part + 6 * kProbThreads);   // [warps][K] per-warp top-K lists
+  int *cand_i = reinterpret_cast<int *>(cand_k + (kProbThreads / 32) * kProbMaxPaths);
   // per-tick log_ndtr of the running maximum and of q for one path, shared by
   // neighbouring classes on dense pixels (the path-group partials, unused
   // then, hold the first)
@@ -239,16 +269,30 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob(ProbArgs a) {
   __shared__ float red[kProbThreads / 32];
   __shared__ float pc[kProbMaxPaths], plp[kProbMaxPaths], nc[kProbMaxPaths], nlp[kProbMaxPaths];
   __shared__ int pskip[kProbMaxPaths];
-  __shared__ int n_cls;
+  __shared__ float slot_c[kProbMaxPaths];       // charge whose values a slot of the scratch holds
+  __shared__ int path_slot[kProbMaxPaths], fresh[kProbMaxPaths];
+  __shared__ int n_cls, n_all, n_fresh, n_slots, stop, again;
+  __shared__ int64_t next_pix;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 
   const LsimParams &p = a.p;
   const int T = a.T, K = a.K, H = p.max_adc_values, tid = threadIdx.x;
   const float z = a.z, thr = a.thr;
   const float term_m1 = ldn_log_term(-1.0f);
+  const float log_k = logf((float)K) + 1e-3f;
+  float *cache = a.cache + (size_t)blockIdx.x * K * kCacheArrays * kProbMaxT;
+  auto kept = [&](int slot, int what) { return cache + (size_t)(slot * kCacheArrays + what) * kProbMaxT; };
   auto shifted = [&](int t) { return min(t + a.interval + 1, T - 1); };
+  // the hit term of a path at tick t from its two log_ndtr values and its dist term
+  auto hit_term = [&](int t, float zqs, float zq0, float LQs, float LQ0, float lg) {
+    float le = log_diff_ndtr_f(zqs, zq0, LQs, LQ0, term_m1);
+    le = fminf(le, lg);
+    le = kProbFloor + softplus_f(le - kProbFloor);
+    return sw[t] * le + (1.0f - sw[t]) * kProbFloor;
+  };
 
-  for (int64_t pix = blockIdx.x; pix < a.n_pix; pix += gridDim.x) {
+  bool leave_out = !kDist && !a.all_steps;
+  for (int64_t pix = blockIdx.x; pix < a.n_pix;) {
     const float *w = a.wfs + pix * T;
     for (int t = tid; t < T; t += kProbThreads) qs[t] = w[t] * p.t_sampling;
     __syncthreads();
@@ -257,6 +301,21 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob(ProbArgs a) {
     __syncthreads();
     block_scan_row<kScanMax>(cm, T, red);
     block_scan_row<kScanSuffixMax>(cr, T, red);
+    // rounding of (cm - c) - thr, times z, on both sides of a rise
+    float most = fabsf(thr);
+    if (!kDist) {
+      float m = 0.0f;
+      for (int t = tid; t < T; t += kProbThreads) m = fmaxf(m, isfinite(qs[t]) ? fabsf(qs[t]) : INFINITY);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      if (lane == 0) red[wid] = m;
+      __syncthreads();
+      for (int w2 = 0; w2 < kProbThreads / 32; ++w2) m = fmaxf(m, red[w2]);
+      most += m;
+      __syncthreads();
+    }
+    const bool partial = leave_out && isfinite(most);
+    const float rise = kWeakRise - most * z * (12000.0f / 16777216.0f);
     // esperance values, soft-where weights and the tick classes
     for (int t = tid; t < T - 1; t += kProbThreads) {
       const int s = shifted(t);
@@ -273,85 +332,188 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob(ProbArgs a) {
                ne(qs[s], qs[sp]) || ne(qs[s1], qs[sp1]) || ne(cr[fe], cr[fep]);
       }
       vh[t] = head ? 1.0f : 0.0f;
+      if (!kDist) {   // heads of the classes that count (a class's ticks have one rise)
+        const bool weak = partial && (cm[t + 1] - cm[t]) * z * 1000.0f < rise;
+        vd[t] = weak ? 1.0f : 0.0f;
+        vs[t] = head && !weak ? 1.0f : 0.0f;
+      }
     }
     __syncthreads();
     block_scan_row<kScanSum>(vh, T - 1, red);   // integer counts, exact in float32
+    if (!kDist) block_scan_row<kScanSum>(vs, T - 1, red);
     for (int t = tid; t < T - 1; t += kProbThreads) {
-      const int u = (int)vh[t] - 1;
-      cls[t] = u;
-      if (t == 0 || (int)vh[t - 1] != u + 1) rep[u] = t;
-      if (t == T - 2) n_cls = u + 1;
+      const bool first = t == 0 || vh[t - 1] != vh[t];
+      const int u = (int)(kDist ? vh[t] : vs[t]) - 1;
+      const bool weak = !kDist && vd[t] != 0.0f;
+      cls[t] = weak ? -1 : u;
+      if (first && !weak) rep[u] = t;
+      if (t == T - 2) {
+        n_cls = u + 1;
+        n_all = (int)vh[t];
+      }
     }
     if (tid < K) {
       pc[tid] = 0.0f;
       plp[tid] = tid == 0 ? 0.0f : kProbFloor;
     }
+    if (tid == 0) {
+      n_slots = 0;
+      stop = 0;
+      again = 0;
+    }
     __syncthreads();
     const int U = n_cls;
     // with few classes, G groups of threads share a class and split the paths
-    const int G = U <= kProbThreads / 2 ? min(8, kProbThreads / U) : 1;
-    const int grp = G > 1 ? tid / U : 0;
+    // (by all classes' number: the order of a class's sum does not depend on what is left out)
+    const int G = n_all <= kProbThreads / 2 ? min(8, kProbThreads / n_all) : 1;
+    const int grp = G > 1 && U > 0 ? tid / U : 0;
     const int n_own = G > 1 ? (grp < G ? 1 : 0) : kProbTicks;
     const int r0 = G > 1 ? tid - grp * U : tid;
     // dense pixels: per path, log_ndtr at every tick (2 T calls) instead of
     // four per class (the running maximum at t + 1 and q at the shifted tick
     // are other ticks' values at t)
-    const bool tick_mode = G == 1 && 2 * U > T;
+    const bool tick_mode = kDist && G == 1 && 2 * U > T;
 
-    for (int h = 0; h < H; ++h) {
+    int h = 0;
+    for (; h < H; ++h) {
       // paths whose charge repeats that of a path more than 110 log units
       // likelier add exp(< -110) = 0 to every float32 log-sum-exp: skip them
-      if (tid < K) {
-        int sk = 0;
-        for (int j = 0; j < K; ++j)
-          if (j != tid && pc[j] == pc[tid] && plp[j] > plp[tid] + 110.0f) sk = 1;
-        pskip[tid] = sk;
-        if (a.state) {
-          float *st = a.state + ((pix * H + h) * 2) * (int64_t)K;
-          st[tid] = pc[tid];
-          st[K + tid] = plp[tid];
+      if (wid == 0) {
+        const float c = lane < K ? pc[lane] : 0.0f;
+        if (lane < K) {
+          int sk = 0;
+          for (int j = 0; j < K; ++j)
+            if (j != lane && pc[j] == c && plp[j] > plp[lane] + 110.0f) sk = 1;
+          pskip[lane] = sk;
+          if (a.state) {
+            float *st = a.state + ((pix * H + h) * 2) * (int64_t)K;
+            st[lane] = c;
+            st[K + lane] = plp[lane];
+          }
+        }
+        // slots: a charge that a slot holds keeps it, the others (one per
+        // distinct charge) take the slots that are free
+        const unsigned key = __float_as_uint(c);
+        int slot = -1;
+        for (int j = 0; j < n_slots; ++j)
+          if (lane < K && __float_as_uint(slot_c[j]) == key) slot = j;
+        const unsigned same = __match_any_sync(0xffffffffu, lane < K ? (unsigned long long)key
+                                                                     : (1ull << 32) + (unsigned)lane);
+        const int leader = __ffs(same) - 1;
+        const unsigned used = __reduce_or_sync(0xffffffffu, slot >= 0 ? 1u << slot : 0u);
+        const unsigned need = __ballot_sync(0xffffffffu, lane < K && slot < 0 && leader == lane);
+        const int rank = __popc(need & ((1u << lane) - 1u));
+        if ((need >> lane) & 1u) {
+          unsigned free_slots = ~used;
+          for (int j = 0; j < rank; ++j) free_slots &= free_slots - 1;
+          slot = __ffs(free_slots) - 1;
+          fresh[rank] = lane;
+        }
+        slot = __shfl_sync(0xffffffffu, slot, leader);
+        __syncwarp();
+        if (lane < K) {
+          path_slot[lane] = slot;
+          slot_c[slot] = c;
+        }
+        const int top = __reduce_max_sync(0xffffffffu, lane < K ? slot + 1 : 0);
+        if (lane == 0) {
+          n_fresh = __popc(need);
+          n_slots = max(n_slots, top);   // a slot that is not in use keeps its charge's values until it is taken
         }
       }
+      __syncthreads();
+      // ---- the values of the charges that are new
+      const int nf = n_fresh;
+      auto evaluate = [&](int r, float c, float *kd, float *ks, float *kh) {
+        const int t = rep[r];
+        const int s = shifted(t);
+        const float zm0 = ((cm[t] - c) - thr) * z, zm1 = ((cm[t + 1] - c) - thr) * z;
+        const float LM0 = tick_mode ? lmv[t] : log_ndtr_f(zm0);
+        const float LM1 = tick_mode ? lmv[t + 1] : (zm1 == zm0 ? LM0 : log_ndtr_f(zm1));
+        const float lg = log_diff_ndtr_f(zm1, zm0, LM1, LM0, term_m1);
+        kd[r] = lg;
+        const int fe = min(s + a.interval + 1, T - 1);
+        const float x = (((cr[fe] - c) - (qs[min(s + 1, T - 1)] - c)) - thr) * z;
+        ks[r] = lg + log_ndtr_f(x);
+        if (kDist) {
+          const float zq0 = ((qs[t] - c) - thr) * z, zqs = ((qs[s] - c) - thr) * z;
+          const float LQ0 = tick_mode ? lqv[t] : log_ndtr_f(zq0);
+          const float LQs = tick_mode ? lqv[s] : (zqs == zq0 ? LQ0 : log_ndtr_f(zqs));
+          kh[r] = hit_term(t, zqs, zq0, LQs, LQ0, lg);
+        } else {
+          kh[r] = kNoHit;
+        }
+      };
+      if (kDist) {
+        for (int f = grp; n_own > 0 && f < nf; f += G) {
+          const int k = fresh[f];
+          const float c = pc[k];
+          float *kd = kept(path_slot[k], 0), *ks = kept(path_slot[k], 1), *kh = kept(path_slot[k], 2);
+          if (tick_mode) {
+            __syncthreads();   // the previous path's reads are done
+            for (int t = tid; t < T; t += kProbThreads) {
+              lmv[t] = log_ndtr_f(((cm[t] - c) - thr) * z);
+              lqv[t] = log_ndtr_f(((qs[t] - c) - thr) * z);
+            }
+            __syncthreads();
+          }
+#pragma unroll
+          for (int i = 0; i < kProbTicks; ++i) {
+            const int r = r0 + i * kProbThreads;
+            if (i < n_own && r < U) evaluate(r, c, kd, ks, kh);
+          }
+        }
+      } else {
+        // (path, class) pairs dealt over all threads
+        int f = 0, r = tid;
+        for (;; r += kProbThreads) {
+          while (r >= U && f < nf) r -= U, ++f;
+          if (f >= nf) break;
+          const int k = fresh[f], slot = path_slot[k];
+          evaluate(r, pc[k], kept(slot, 0), kept(slot, 1), kept(slot, 2));
+        }
+      }
+      __syncthreads();
+      // ---- the log-sum-exps over the paths
       float hm[kProbTicks], hs[kProbTicks], dm[kProbTicks], ds[kProbTicks], sm_[kProbTicks], ss[kProbTicks];
 #pragma unroll
       for (int i = 0; i < kProbTicks; ++i) {
         hm[i] = dm[i] = sm_[i] = -INFINITY;
         hs[i] = ds[i] = ss[i] = 0.0f;
       }
-      __syncthreads();
       for (int k = grp; n_own > 0 && k < K; k += G) {
         if (pskip[k]) continue;
         const float c = pc[k], lp = plp[k];
-        if (tick_mode) {
-          __syncthreads();   // the previous path's reads are done
-          for (int t = tid; t < T; t += kProbThreads) {
-            lmv[t] = log_ndtr_f(((cm[t] - c) - thr) * z);
-            lqv[t] = log_ndtr_f(((qs[t] - c) - thr) * z);
-          }
-          __syncthreads();
+        const float *kd = kept(path_slot[k], 0), *ks = kept(path_slot[k], 1);
+        float *kh = kept(path_slot[k], 2);
+        float lg[kProbTicks], lsel[kProbTicks], le[kProbTicks];
+#pragma unroll
+        for (int i = 0; i < kProbTicks; ++i) {
+          const int r = r0 + i * kProbThreads;
+          const bool ok = i < n_own && r < U;
+          lg[i] = ok ? kd[r] : 0.0f;
+          lsel[i] = ok ? ks[r] : 0.0f;
+          le[i] = ok ? kh[r] : 0.0f;
         }
 #pragma unroll
         for (int i = 0; i < kProbTicks; ++i) {
           const int r = r0 + i * kProbThreads;
           if (i < n_own && r < U) {
-            const int t = rep[r];
-            const int s = shifted(t);
-            const float zm0 = ((cm[t] - c) - thr) * z, zm1 = ((cm[t + 1] - c) - thr) * z;
-            const float LM0 = tick_mode ? lmv[t] : log_ndtr_f(zm0);
-            const float LM1 = tick_mode ? lmv[t + 1] : (zm1 == zm0 ? LM0 : log_ndtr_f(zm1));
-            const float lg = log_diff_ndtr_f(zm1, zm0, LM1, LM0, term_m1);
-            const float zq0 = ((qs[t] - c) - thr) * z, zqs = ((qs[s] - c) - thr) * z;
-            const float LQ0 = tick_mode ? lqv[t] : log_ndtr_f(zq0);
-            const float LQs = tick_mode ? lqv[s] : (zqs == zq0 ? LQ0 : log_ndtr_f(zqs));
-            float le = log_diff_ndtr_f(zqs, zq0, LQs, LQ0, term_m1);
-            le = fminf(le, lg);
-            le = kProbFloor + softplus_f(le - kProbFloor);
-            le = sw[t] * le + (1.0f - sw[t]) * kProbFloor;
-            lse_add(hm[i], hs[i], le + lp);
-            lse_add(dm[i], ds[i], lg + lp);
-            const int fe = min(s + a.interval + 1, T - 1);
-            const float x = (((cr[fe] - c) - (qs[min(s + 1, T - 1)] - c)) - thr) * z;
-            lse_add(sm_[i], ss[i], (lg + log_ndtr_f(x)) + lp);
+            if (kDist) {
+              lse_add(hm[i], hs[i], le[i] + lp);
+            } else if (!(lg[i] + lp < kProbFar)) {
+              if (le[i] == kNoHit) {
+                const int t = rep[r], s = shifted(t);
+                const float zq0 = ((qs[t] - c) - thr) * z, zqs = ((qs[s] - c) - thr) * z;
+                const float LQ0 = log_ndtr_f(zq0);
+                const float LQs = zqs == zq0 ? LQ0 : log_ndtr_f(zqs);
+                le[i] = hit_term(t, zqs, zq0, LQs, LQ0, lg[i]);
+                kh[r] = le[i];
+              }
+              lse_add(hm[i], hs[i], le[i] + lp);
+            }
+            lse_add(dm[i], ds[i], lg[i] + lp);
+            lse_add(sm_[i], ss[i], lsel[i] + lp);
           }
         }
       }
@@ -384,89 +546,123 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob(ProbArgs a) {
       // step outputs and the per-hit reductions
       float l_sum = 0.0f, t_sum = 0.0f, a_sum = 0.0f;
       float selv[kProbTicks];
+      unsigned left = 0u;     // this thread's ticks that are not in the selection
       const int64_t row = (pix * H + h) * (int64_t)(T - 1);
 #pragma unroll
       for (int i = 0; i < kProbTicks; ++i) {
         const int t = tid + i * kProbThreads;
         selv[i] = -INFINITY;
-        if (t < T - 1) {
-          const int u = cls[t];
+        float pr = 0.0f;
+        const int u = t < T - 1 ? cls[t] : -1;
+        if (u < 0) left |= 1u << i;
+        if (u >= 0) {
           const float hit = vh[u];
           selv[i] = vs[u];
           if (a.log_prob) a.log_prob[row + t] = hit;
           if (a.charge) a.charge[row + t] = esp[t];
-          const float pr = expf(hit);
+          pr = expf(hit);
           l_sum += pr;
           t_sum += (float)t * pr;
           a_sum += digitize(p, esp[t]) * pr;
         }
+        if (a.live) {   // NaN counts as live
+          const unsigned bits = __ballot_sync(0xffffffffu, pr != 0.0f);
+          if (lane == 0) a.live[(pix * H + h) * kLiveWords + i * (kProbThreads / 32) + wid] = bits;
+        }
       }
-      if (a.lam) {
+      if (a.lam || a.red) {
         const float L = block_sum(l_sum, red);
         const float Ts = block_sum(t_sum, red);
         const float As = block_sum(a_sum, red);
         if (tid == 0) {
-          const float den = fmaxf(L, 1e-10f);
-          a.lam[pix * H + h] = L;
-          a.e_tick[pix * H + h] = Ts / den;
-          a.e_adc[pix * H + h] = As / den;
+          const float den = fmaxf(L, 1e-10f), et = Ts / den, ea = As / den;
+          const int64_t o = pix * H + h;
+          if (a.lam) {
+            a.lam[o] = L;
+            a.e_tick[o] = et;
+            a.e_adc[o] = ea;
+          }
+          if (a.red) {
+            a.red[o] = et;
+            a.red[a.n_pix * H + o] = ea;
+            a.red[2 * a.n_pix * H + o] = L;
+          }
         }
       }
-      // top-K ticks by selection value -> next paths: each warp keeps the K
-      // best of its ticks (largest first, lower tick first on ties), then
-      // warp 0 takes the K best of those candidates
+      // top-K ticks by selection value -> next paths (largest first, lower tick
+      // first on ties, NaN never): each warp lists the K best of its ticks,
+      // then warp 0 merges the 16 lists.  The values are compared as ordered
+      // integers, so a round is two warp reductions.
       {
-        unsigned taken = 0;
-        for (int r = 0; r < K; ++r) {
-          float bv = -INFINITY;
-          int bi = 0x7fffffff;
+        unsigned key[kProbTicks];
 #pragma unroll
-          for (int i = 0; i < kProbTicks; ++i) {
-            const int t = tid + i * kProbThreads;
-            if (t < T - 1 && !(taken >> i & 1u) && better(selv[i], t, bv, bi)) {
-              bv = selv[i];
-              bi = t;
+        for (int i = 0; i < kProbTicks; ++i)
+          key[i] = (left >> i & 1u) || selv[i] != selv[i] ? 0u : order_key(selv[i]);
+        unsigned mine_k = 0u;
+        int mine_t = 0x7fffffff;
+        for (int r = 0; r < K; ++r) {
+          unsigned bk = 0u;
+          int bi = 0;
+#pragma unroll
+          for (int i = 0; i < kProbTicks; ++i)
+            if (key[i] > bk) {
+              bk = key[i];
+              bi = i;
             }
+          const unsigned m = __reduce_max_sync(0xffffffffu, bk);
+          if (m == 0u) break;
+          const int t = tid + bi * kProbThreads;
+          const int first = __reduce_min_sync(0xffffffffu, bk == m ? t : 0x7fffffff);
+          if (t == first)
+#pragma unroll
+            for (int i = 0; i < kProbTicks; ++i)
+              if (i == bi) key[i] = 0u;
+          if (lane == r) {
+            mine_k = m;
+            mine_t = first;
           }
-          warp_best(bv, bi);
-          if (bi != 0x7fffffff && (bi % kProbThreads) == tid) taken |= 1u << (bi / kProbThreads);
-          if (lane == 0) {
-            cand_v[wid * kProbMaxPaths + r] = bv;
-            cand_i[wid * kProbMaxPaths + r] = bi;
-          }
+        }
+        if (lane < K) {
+          cand_k[wid * kProbMaxPaths + lane] = mine_k;
+          cand_i[wid * kProbMaxPaths + lane] = mine_t;
         }
       }
       __syncthreads();
       if (wid == 0) {
-        constexpr int kCand = (kProbThreads / 32) * kProbMaxPaths / 32;   // candidates per lane
-        float cv[kCand];
-        int ci[kCand];
-#pragma unroll
-        for (int j = 0; j < kCand; ++j) {
-          const int e = lane + 32 * j, w2 = e / kProbMaxPaths, r2 = e % kProbMaxPaths;
-          cv[j] = r2 < K ? cand_v[w2 * kProbMaxPaths + r2] : -INFINITY;
-          ci[j] = r2 < K ? cand_i[w2 * kProbMaxPaths + r2] : 0x7fffffff;
-        }
-        unsigned taken = 0;
+        static_assert(kProbThreads / 32 <= 32, "a lane per list");
+        const int base = lane * kProbMaxPaths;
+        const bool list = lane < kProbThreads / 32;
+        int at = 0, tt = 0x7fffffff;
+        unsigned hk = list ? cand_k[base] : 0u, bv = 0u;
+        int hi = list ? cand_i[base] : 0x7fffffff;
         for (int r = 0; r < K; ++r) {
-          float bv = -INFINITY;
-          int bi = 0x7fffffff, bj = -1;
-#pragma unroll
-          for (int j = 0; j < kCand; ++j)
-            if (!(taken >> j & 1u) && better(cv[j], ci[j], bv, bi)) {
-              bv = cv[j];
-              bi = ci[j];
-              bj = j;
-            }
-          const int mine = bi;
-          warp_best(bv, bi);
-          if (bj >= 0 && mine == bi) taken |= 1u << bj;
+          const unsigned m = __reduce_max_sync(0xffffffffu, hk);
+          if (m == 0u) break;
+          const int first = __reduce_min_sync(0xffffffffu, hk == m ? hi : 0x7fffffff);
           if (lane == r) {
-            const int tt = bi >= 0 && bi < T - 1 ? bi : T - 2;
-            nlp[r] = vd[cls[tt]];
-            nc[r] = qs[min(shifted(tt) + 1, T - 1)];
-            if (a.state_top) a.state_top[(pix * H + h) * (int64_t)K + r] = tt;
+            bv = m;
+            tt = first;
           }
+          if (hk == m && hi == first) {
+            ++at;
+            hk = at < K ? cand_k[base + at] : 0u;
+            hi = at < K ? cand_i[base + at] : 0x7fffffff;
+          }
+        }
+        // charge of the paths that are missing, and what a tick left out can at most be selected by
+        const int best = __shfl_sync(0xffffffffu, tt, 0);
+        const float miss_c = best < T - 1 ? qs[min(shifted(best) + 1, T - 1)] : 0.0f;
+        float mp = lane < K ? plp[lane] : -INFINITY;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mp = fmaxf(mp, __shfl_xor_sync(0xffffffffu, mp, o));
+        if (lane < K) {
+          const bool have = tt < T - 1, real = have || !partial;
+          if (!have) tt = T - 2;
+          const float lp_new = real ? vd[cls[tt]] : kProbFloor;
+          nlp[lane] = lp_new;
+          nc[lane] = real ? qs[min(shifted(tt) + 1, T - 1)] : miss_c;
+          if (partial && have && !(key_order(bv) > mp + log_k + kWeakMost) && !(lp_new < kProbFar)) again = 1;
+          if (a.state_top) a.state_top[(pix * H + h) * (int64_t)K + lane] = tt;
         }
       }
       __syncthreads();
@@ -483,11 +679,38 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob(ProbArgs a) {
           pc[tid] = nc[tid];
           plp[tid] = nlp[tid];
         }
-        if (tid == 0 && logf(sum) + mm > a.log_stop && !*(volatile int32_t *)(a.step_active + h))
-          atomicOr(a.step_active + h, 1);
+        if (tid == 0) {
+          const float total = logf(sum) + mm;
+          if (!again && total > a.log_stop && !*(volatile int32_t *)(a.step_active + h)) atomicOr(a.step_active + h, 1);
+          // a step at most multiplies the total by K (its K ticks' dist values)
+          stop = partial && total < kProbDead - 1.0f - log_k * (float)(H - 1 - h) ? 1 : 0;
+        }
       }
       __syncthreads();
+      if (again) break;
+      if (stop) {
+        ++h;
+        break;
+      }
     }
+    if (again) {        // once more with every class
+      leave_out = false;
+      __syncthreads();
+      continue;
+    }
+    if (a.n_run && tid == 0) a.n_run[pix] = h;
+    // the steps that were not run: every probability is exactly 0
+    for (int g = h + tid; g < H; g += kProbThreads)
+      if (a.lam) {
+        a.lam[pix * H + g] = 0.0f;
+        a.e_tick[pix * H + g] = 0.0f;
+        a.e_adc[pix * H + g] = 0.0f;
+      }
+    leave_out = !kDist && !a.all_steps;
+    // pixels differ several times in cost: the next one by a counter
+    if (tid == 0) next_pix = gridDim.x + (int64_t)atomicAdd(a.work, 1ull);
+    __syncthreads();
+    pix = next_pix;
   }
 }
 
@@ -563,7 +786,7 @@ __device__ __forceinline__ float ldn_grad(float a, float b, float la, float lb, 
 }
 
 struct ProbVjpArgs {
-  ProbArgs f;                  // the forward's arguments (state, state_top, step_active read)
+  ProbArgs f;                  // the forward's arguments (its record, step_active and reductions read)
   const float *g_log_prob;     // optional [n_pix][H][T-1]
   const float *g_charge;       // optional [n_pix][H][T-1]
   const float *g_e_tick, *g_e_adc, *g_lam;   // optional [n_pix][H] (all three or none)
@@ -578,27 +801,32 @@ struct ProbVjpArgs {
 // value) enter linearly, so the partials are evaluated once per class and
 // path, folded into seven per-class coefficients, and spread back to the
 // class's ticks with the ticks' own cotangents.  Classes are also cut at
-// every kVjpSpan ticks, so the per-class loops over ticks stay short (flat
-// stretches of a waveform are long).
+// every kVjpSpan ticks, so a warp's lanes hold a class's ticks.
+//
+// Few classes of a step have a cotangent at all: those of the K selected
+// ticks and those whose probability is not 0 (the forward's record says
+// which), about 5 % of the ticks.  A step lists them, and the 16 warps take
+// one class at a time, lane k for path k: the log-sum-exps, the partials'
+// sums over the paths and the class's ticks are all within a warp.  (A thread
+// per class, walking the K paths, left one or two warps of a block at work
+// and recomputed every class's log-sum-exps: 1500 rows took 16.1 ms.)
 constexpr int kVjpSpan = 16;
-constexpr int kVjpArrays = 13;   // q, running max, 5 accumulators, dist and hit cotangents, class hit and
-                                 // dist values (the hit values double as scratch), class, representative;
-                                 // the esperance and the soft-where weight are recomputed from q, so two
-                                 // blocks fit on an SM
+constexpr int kVjpArrays = 12;   // q, running max, 5 accumulators, dist cotangents, scratch, class, representative,
+                                 // list of live classes; the esperance and the soft-where weight are recomputed from
+                                 // q, so two blocks fit on an SM
 
 __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va) {
   extern __shared__ __align__(16) float sm[];
   const ProbArgs &a = va.f;
   float *qs = sm, *cm = qs + kProbMaxT;
   float *Aq0 = cm + kProbMaxT, *Aqs = Aq0 + kProbMaxT, *Am0 = Aqs + kProbMaxT, *Am1 = Am0 + kProbMaxT;
-  float *Aesp = Am1 + kProbMaxT, *Gd = Aesp + kProbMaxT, *Gh = Gd + kProbMaxT;
-  float *vh = Gh + kProbMaxT, *vd = vh + kProbMaxT;
-  float *tmp = vh;   // scratch before and after the steps, when the class values are not in use
-  int *cls = reinterpret_cast<int *>(vd + kProbMaxT), *rep = cls + kProbMaxT;
-  float *part = reinterpret_cast<float *>(rep + kProbMaxT);   // [warps][2][kProbMaxPaths]
+  float *Aesp = Am1 + kProbMaxT, *Gd = Aesp + kProbMaxT, *tmp = Gd + kProbMaxT;
+  int *cls = reinterpret_cast<int *>(tmp + kProbMaxT), *rep = cls + kProbMaxT, *list = rep + kProbMaxT;
+  float *part = reinterpret_cast<float *>(list + kProbMaxT);   // [warps][2][kProbMaxPaths]
   __shared__ float red[kProbThreads / 32];
   __shared__ float pc[kProbMaxPaths], plp[kProbMaxPaths], glp_n[kProbMaxPaths], gc_n[kProbMaxPaths];
   __shared__ int pskip[kProbMaxPaths], ptop[kProbMaxPaths];
+  __shared__ int counts[kProbTicks][kProbThreads / 32];
   __shared__ int n_exec, n_cls;
 
   const LsimParams &p = a.p;
@@ -619,7 +847,9 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
       }
     n_exec = first;
   }
+  __syncthreads();
 
+  // the record is only read here: backward passes may share it
   for (int64_t pix = blockIdx.x; pix < a.n_pix; pix += gridDim.x) {
     const float *w = a.wfs + pix * T;
     for (int t = tid; t < T; t += kProbThreads) qs[t] = w[t] * p.t_sampling;
@@ -658,21 +888,23 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
     const int U = n_cls;
     if (tid == 0) rep[U] = T - 1;     // end of the last class
 
-    for (int h = n_exec - 1; h >= 0; --h) {
+    for (int h = min(n_exec, a.n_run[pix]) - 1; h >= 0; --h) {
+      const int64_t o = pix * H + h;
       // step h's input paths and selected ticks, recorded by the forward
       if (tid < K) {
-        const float *st = a.state + ((pix * H + h) * 2) * (int64_t)K;
+        const float *st = a.state + (o * 2) * (int64_t)K;
         pc[tid] = st[tid];
         plp[tid] = st[K + tid];
-        ptop[tid] = a.state_top[(pix * H + h) * (int64_t)K + tid];
+        ptop[tid] = a.state_top[o * (int64_t)K + tid];
       }
-      for (int t = tid; t < T; t += kProbThreads) Gd[t] = 0.f;
+      for (int t = tid; t < T; t += kProbThreads) Gd[t] = tmp[t] = 0.f;
       __syncthreads();
       if (tid < K) {
         int sk = 0;
         for (int j = 0; j < K; ++j)
           if (j != tid && pc[j] == pc[tid] && plp[j] > plp[tid] + 110.0f) sk = 1;
         pskip[tid] = sk;
+        if (glp_n[tid] != 0.f) tmp[cls[ptop[tid]]] = 1.f;   // the class has a dist cotangent
       }
       if (tid == 0) {
         // the next step's state cotangents: new lp_j = dist[top_j], new c_j = q[best_j]
@@ -682,165 +914,122 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
           Aq0[min(shifted(tt) + 1, T - 1)] += gc_n[j];
         }
       }
+      if (va.g_charge)
+        for (int t = tid; t < T - 1; t += kProbThreads) Aesp[t] += va.g_charge[o * (int64_t)(T - 1) + t];
       __syncthreads();
-      // ---- pass 1: hit and dist log-sum-exps per class
+      // ---- the classes with a cotangent, in order
+      unsigned live_bits[kProbTicks];
 #pragma unroll
       for (int i = 0; i < kProbTicks; ++i) {
         const int u = tid + i * kProbThreads;
+        bool live = false;
         if (u < U) {
-          float hm = -INFINITY, hs = 0.f, dm = -INFINITY, ds = 0.f;
           const int t = rep[u];
-          const int sidx = shifted(t);
-          const float swt = sw_at(esp_at(t));
-          for (int k = 0; k < K; ++k) {
-            if (pskip[k]) continue;
-            const float c = pc[k], lp = plp[k];
-            const float zm0 = ((cm[t] - c) - thr) * z, zm1 = ((cm[t + 1] - c) - thr) * z;
-            const float LM0 = log_ndtr_f(zm0);
-            const float LM1 = zm1 == zm0 ? LM0 : log_ndtr_f(zm1);
-            const float lg = log_diff_ndtr_f(zm1, zm0, LM1, LM0, term_m1);
-            const float zq0 = ((qs[t] - c) - thr) * z, zqs = ((qs[sidx] - c) - thr) * z;
-            const float LQ0 = log_ndtr_f(zq0);
-            const float LQs = zqs == zq0 ? LQ0 : log_ndtr_f(zqs);
-            float le = log_diff_ndtr_f(zqs, zq0, LQs, LQ0, term_m1);
-            le = fminf(le, lg);
-            le = kProbFloor + softplus_f(le - kProbFloor);
-            le = swt * le + (1.0f - swt) * kProbFloor;
-            lse_add(hm, hs, le + lp);
-            lse_add(dm, ds, lg + lp);
-          }
-          vh[u] = lse_final(hm, hs);
-          vd[u] = lse_final(dm, ds);
+          live = tmp[u] != 0.f;
+          if (va.g_lam && !live) live = (a.live[o * kLiveWords + (t >> 5)] >> (t & 31)) & 1u;
+          if (va.g_log_prob)
+            for (int tt = t; tt < rep[u + 1] && !live; ++tt) live = va.g_log_prob[o * (int64_t)(T - 1) + tt] != 0.f;
         }
+        live_bits[i] = __ballot_sync(0xffffffffu, live);
+        if (lane == 0) counts[i][wid] = __popc(live_bits[i]);
       }
       __syncthreads();
-      // ---- cotangents of the step's outputs on each tick
-      float l_sum = 0.f, t_sum = 0.f, a_sum = 0.f;
-      float pr[kProbTicks];
-#pragma unroll
-      for (int i = 0; i < kProbTicks; ++i) {
-        const int t = tid + i * kProbThreads;
-        pr[i] = 0.f;
-        if (t < T - 1) {
-          const int64_t o = (pix * H + h) * (int64_t)(T - 1) + t;
-          Gh[t] = va.g_log_prob ? va.g_log_prob[o] : 0.f;
-          if (va.g_charge) Aesp[t] += va.g_charge[o];
-          pr[i] = expf(vh[cls[t]]);
-          l_sum += pr[i];
-          t_sum += (float)t * pr[i];
-          a_sum += digitize(p, esp_at(t)) * pr[i];
-        }
-      }
-      if (va.g_lam) {
-        const float L = block_sum(l_sum, red);
-        const float Ts = block_sum(t_sum, red);
-        const float As = block_sum(a_sum, red);
-        const float den = fmaxf(L, 1e-10f);
-        const float on = L > 1e-10f ? 1.f : (L == 1e-10f ? 0.5f : 0.f);   // jnp.maximum's share
-        const float ET = Ts / den, EA = As / den;
-        const int64_t o = pix * H + h;
-        const float gl = va.g_lam[o], gt = va.g_e_tick[o], ga = va.g_e_adc[o];
-        // the lambda cotangent also reaches ET and EA through the denominator
-        const float gden = -(gt * ET + ga * EA) / den;
-#pragma unroll
-        for (int i = 0; i < kProbTicks; ++i) {
-          const int t = tid + i * kProbThreads;
-          if (t < T - 1) {
-            const float et = esp_at(t);
-            const float adc = digitize(p, et);
-            const float gp = gl + gt * (float)t / den + ga * adc / den + on * gden;
-            Gh[t] += gp * pr[i];
-            Aesp[t] += digitize_vjp(p, et, ga * pr[i] / den);
-          }
-        }
-      }
-      __syncthreads();
-      // ---- per class: sums of the ticks' cotangents
-      float Hs[kProbTicks], Ds[kProbTicks];
-      bool anyH[kProbTicks], anyD[kProbTicks];
-#pragma unroll
-      for (int i = 0; i < kProbTicks; ++i) {
-        const int u = tid + i * kProbThreads;
-        Hs[i] = Ds[i] = 0.f;
-        anyH[i] = anyD[i] = false;
-        if (u < U)
-          for (int t = rep[u]; t < rep[u + 1]; ++t) {
-            const float gh = Gh[t], gd = Gd[t];
-            Hs[i] += gh;
-            Ds[i] += gd;
-            anyH[i] |= gh != 0.f;
-            anyD[i] |= gd != 0.f;
-          }
-      }
-      // ---- pass 2: the partials per class and path, folded into seven
-      // per-class coefficients of the ticks' (hit, dist) cotangents
-      float co[kProbTicks][7];
+      int n_live = 0;
 #pragma unroll
       for (int i = 0; i < kProbTicks; ++i)
+        for (int w2 = 0; w2 < kProbThreads / 32; ++w2) {
+          if (w2 == wid && (live_bits[i] >> lane) & 1u)
+            list[n_live + __popc(live_bits[i] & ((1u << lane) - 1u))] = tid + i * kProbThreads;
+          n_live += counts[i][w2];
+        }
+      __syncthreads();
+      // the reductions' cotangents, common to the step's ticks
+      float gl = 0.f, gt = 0.f, ga = 0.f, den = 1.f;
+      if (va.g_lam) {
+        const float ET = a.red[o], EA = a.red[a.n_pix * H + o], L = a.red[2 * a.n_pix * H + o];
+        den = fmaxf(L, 1e-10f);
+        const float on = L > 1e-10f ? 1.f : (L == 1e-10f ? 0.5f : 0.f);   // jnp.maximum's share
+        gt = va.g_e_tick[o];
+        ga = va.g_e_adc[o];
+        // the lambda cotangent also reaches ET and EA through the denominator
+        gl = va.g_lam[o] + on * (-(gt * ET + ga * EA) / den);
+      }
+      const bool path = lane < K && !pskip[lane < K ? lane : 0];
+      const float c = lane < K ? pc[lane] : 0.f, lp = lane < K ? plp[lane] : 0.f;
+      float glp = 0.f, gc = 0.f;      // lane k: path k's cotangents
+      for (int e = wid; e < n_live; e += kProbThreads / 32) {
+        const int u = list[e], t = rep[u], nt = rep[u + 1] - t;
+        const int sidx = shifted(t);
+        // ---- lane k: path k's values and partials at the class
+        const float zm0 = ((cm[t] - c) - thr) * z, zm1 = ((cm[t + 1] - c) - thr) * z;
+        const float LM0 = log_ndtr_f(zm0), LM1 = log_ndtr_f(zm1);
+        float g_m1, g_m0;
+        const float lg = ldn_grad(zm1, zm0, LM1, LM0, dlog_ndtr_f(zm1, LM1), dlog_ndtr_f(zm0, LM0), term_m1, g_m1,
+                                  g_m0);
+        const float zq0 = ((qs[t] - c) - thr) * z, zqs = ((qs[sidx] - c) - thr) * z;
+        const float LQ0 = log_ndtr_f(zq0), LQs = log_ndtr_f(zqs);
+        float g_qs, g_q0;
+        const float lep = ldn_grad(zqs, zq0, LQs, LQ0, dlog_ndtr_f(zqs, LQs), dlog_ndtr_f(zq0, LQ0), term_m1, g_qs,
+                                   g_q0);
+        const float le1 = fminf(lep, lg);
+        const float le2 = kProbFloor + softplus_f(le1 - kProbFloor);
+        const float wt = sw_at(esp_at(t));
+        const float le = wt * le2 + (1.0f - wt) * kProbFloor;
+        // ---- hit and dist log-sum-exps
+        auto lse = [&](float x) {
+          float m = path ? x : -INFINITY;
 #pragma unroll
-        for (int j = 0; j < 7; ++j) co[i][j] = 0.f;
-      for (int k = 0; k < K; ++k) {
-        float glp = 0.f, gc = 0.f;
-        if (!pskip[k]) {
-          const float c = pc[k], lp = plp[k];
-#pragma unroll
-          for (int i = 0; i < kProbTicks; ++i) {
-            const int u = tid + i * kProbThreads;
-            if (u >= U || !(anyH[i] || anyD[i])) continue;
-            const int t = rep[u];
-            const int sidx = shifted(t);
-            const float zm0 = ((cm[t] - c) - thr) * z, zm1 = ((cm[t + 1] - c) - thr) * z;
-            const float LM0 = log_ndtr_f(zm0), LM1 = log_ndtr_f(zm1);
-            float g_m1, g_m0;
-            const float lg = ldn_grad(zm1, zm0, LM1, LM0, dlog_ndtr_f(zm1, LM1), dlog_ndtr_f(zm0, LM0), term_m1,
-                                      g_m1, g_m0);
-            const float zq0 = ((qs[t] - c) - thr) * z, zqs = ((qs[sidx] - c) - thr) * z;
-            const float LQ0 = log_ndtr_f(zq0), LQs = log_ndtr_f(zqs);
-            float g_qs, g_q0;
-            const float lep = ldn_grad(zqs, zq0, LQs, LQ0, dlog_ndtr_f(zqs, LQs), dlog_ndtr_f(zq0, LQ0), term_m1,
-                                       g_qs, g_q0);
-            const float le1 = fminf(lep, lg);
-            const float le2 = kProbFloor + softplus_f(le1 - kProbFloor);
-            const float wt = sw_at(esp_at(t));
-            const float le = wt * le2 + (1.0f - wt) * kProbFloor;
-            // d(hit log-sum-exp)/d(le + lp) and d(dist log-sum-exp)/d(lg + lp)
-            const float al = anyH[i] ? expf((le + lp) - vh[u]) : 0.f;
-            const float be = anyD[i] ? expf((lg + lp) - vd[u]) : 0.f;
-            glp += al * Hs[i] + be * Ds[i];
-            // per unit hit cotangent: le = w le2 + (1 - w)(-1000), w = sigmoid((esp - thr) 10)
-            const float gl1 = al * wt * sigmoid_f(le1 - kProbFloor);
-            const float s_lep = lep < lg ? 1.f : (lep == lg ? 0.5f : 0.f);
-            const float hl = gl1 * s_lep, hg = gl1 * (1.f - s_lep);
-            co[i][0] += hl * g_q0 * z;
-            co[i][1] += hl * g_qs * z;
-            co[i][2] += hg * g_m0 * z;
-            co[i][3] += be * g_m0 * z;
-            co[i][4] += hg * g_m1 * z;
-            co[i][5] += be * g_m1 * z;
-            co[i][6] += al * (le2 - kProbFloor) * wt * (1.0f - wt) * 10.0f;
-            gc -= (Hs[i] * (hl * (g_q0 + g_qs) + hg * (g_m0 + g_m1)) + Ds[i] * be * (g_m0 + g_m1)) * z;
+          for (int s2 = 16; s2 > 0; s2 >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s2));
+          return logf(warp_sum(path ? expf(x - m) : 0.f)) + m;
+        };
+        const float vh = lse(le + lp), vd = lse(lg + lp);
+        // ---- the class's ticks, lane j for its tick j
+        float gh = 0.f, gd = 0.f;
+        if (lane < nt) {
+          const int tt = t + lane;
+          if (va.g_log_prob) gh = va.g_log_prob[o * (int64_t)(T - 1) + tt];
+          gd = Gd[tt];
+          if (va.g_lam) {
+            const float pr = expf(vh), et = esp_at(tt);
+            gh += (gl + gt * (float)tt / den + ga * digitize(p, et) / den) * pr;
+            Aesp[tt] += digitize_vjp(p, et, ga * pr / den);
           }
         }
-        glp = warp_sum(glp);
-        gc = warp_sum(gc);
-        if (lane == 0) {
-          part[(wid * 2) * kProbMaxPaths + k] = glp;
-          part[(wid * 2 + 1) * kProbMaxPaths + k] = gc;
+        const bool any_h = __any_sync(0xffffffffu, gh != 0.f), any_d = __any_sync(0xffffffffu, gd != 0.f);
+        const float Hs = warp_sum(gh), Ds = warp_sum(gd);
+        // d(hit log-sum-exp)/d(le + lp) and d(dist log-sum-exp)/d(lg + lp)
+        const float al = any_h && path ? expf((le + lp) - vh) : 0.f;
+        const float be = any_d && path ? expf((lg + lp) - vd) : 0.f;
+        // per unit hit cotangent: le = w le2 + (1 - w)(-1000), w = sigmoid((esp - thr) 10)
+        const float gl1 = al * wt * sigmoid_f(le1 - kProbFloor);
+        const float s_lep = lep < lg ? 1.f : (lep == lg ? 0.5f : 0.f);
+        const float hl = gl1 * s_lep, hg = gl1 * (1.f - s_lep);
+        float co[7];
+        co[0] = hl * g_q0 * z;
+        co[1] = hl * g_qs * z;
+        co[2] = hg * g_m0 * z;
+        co[3] = be * g_m0 * z;
+        co[4] = hg * g_m1 * z;
+        co[5] = be * g_m1 * z;
+        co[6] = al * (le2 - kProbFloor) * wt * (1.0f - wt) * 10.0f;
+        if (path) {
+          glp += al * Hs + be * Ds;
+          gc -= (Hs * (hl * (g_q0 + g_qs) + hg * (g_m0 + g_m1)) + Ds * be * (g_m0 + g_m1)) * z;
+        }
+#pragma unroll
+        for (int j = 0; j < 7; ++j) co[j] = warp_sum(path ? co[j] : 0.f);
+        if (lane < nt) {
+          const int tt = t + lane;
+          Aq0[tt] += gh * co[0];
+          Aqs[tt] += gh * co[1];
+          Am0[tt] += gh * co[2] + gd * co[3];
+          Am1[tt] += gh * co[4] + gd * co[5];
+          Aesp[tt] += gh * co[6];
         }
       }
-      // spread the coefficients to the class's ticks with their cotangents
-#pragma unroll
-      for (int i = 0; i < kProbTicks; ++i) {
-        const int u = tid + i * kProbThreads;
-        if (u >= U || !(anyH[i] || anyD[i])) continue;
-        for (int t = rep[u]; t < rep[u + 1]; ++t) {
-          const float gh = Gh[t], gd = Gd[t];
-          Aq0[t] += gh * co[i][0];
-          Aqs[t] += gh * co[i][1];
-          Am0[t] += gh * co[i][2] + gd * co[i][3];
-          Am1[t] += gh * co[i][4] + gd * co[i][5];
-          Aesp[t] += gh * co[i][6];
-        }
+      if (lane < K) {
+        part[(wid * 2) * kProbMaxPaths + lane] = glp;
+        part[(wid * 2 + 1) * kProbMaxPaths + lane] = gc;
       }
       __syncthreads();
       if (tid < K) {
@@ -890,14 +1079,56 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
 
 }  // namespace
 
-size_t fee_prob_workspace_bytes(int32_t max_adc_values) {
-  return ((size_t)(max_adc_values > 0 ? max_adc_values : 1) * sizeof(int32_t) + 255) & ~size_t(255);
+// Blocks of the forward kernel: two per SM.
+static int64_t prob_blocks() { return (int64_t)device_sm_count() * 2; }
+
+static size_t al256(size_t b) { return (b + 255) & ~size_t(255); }
+
+// The steps' flags and, at the end of their 256 bytes, the forward's pixel counter.
+constexpr size_t kFlagBytes = 256;
+static_assert(sizeof(int32_t) * LSIM_MAX_HITS + sizeof(unsigned long long) <= kFlagBytes, "flags and counter");
+static unsigned long long *work_counter(int32_t *flags) {
+  return reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(flags) + kFlagBytes) - 1;
 }
 
-static ProbArgs prob_args(const LsimParams &p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
-                          float stop_threshold, float *log_prob, float *charge, float *e_tick, float *e_adc,
-                          float *lam, void *ws) {
-  ProbArgs a;
+// step_active, then the blocks' path values (for any number of paths and pixels)
+size_t fee_prob_workspace_bytes(int32_t) {
+  return kFlagBytes + sizeof(float) * (size_t)prob_blocks() * kProbMaxPaths * kCacheArrays * kProbMaxT;
+}
+
+struct ProbRecord {
+  int32_t *step_active, *n_run, *top;
+  float *state, *red;
+  uint32_t *live;
+};
+
+static size_t record_layout(int64_t n_pix, int32_t max_adc_values, int32_t n_paths, ProbRecord *r, char *base) {
+  const size_t steps = (size_t)(n_pix > 0 ? n_pix : 0) * (size_t)max_adc_values;
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    const size_t at = off;
+    off += al256(bytes);
+    return base ? base + at : nullptr;
+  };
+  char *active = take(kFlagBytes);
+  char *state = take(sizeof(float) * 2 * steps * n_paths);
+  char *top = take(sizeof(int32_t) * steps * n_paths);
+  char *run = take(sizeof(int32_t) * (size_t)(n_pix > 0 ? n_pix : 0));
+  char *live = take(sizeof(uint32_t) * steps * kLiveWords);
+  char *red = take(sizeof(float) * 3 * steps);
+  if (r)
+    *r = ProbRecord{reinterpret_cast<int32_t *>(active), reinterpret_cast<int32_t *>(run),
+                    reinterpret_cast<int32_t *>(top), reinterpret_cast<float *>(state),
+                    reinterpret_cast<float *>(red), reinterpret_cast<uint32_t *>(live)};
+  return off;
+}
+
+size_t fee_prob_record_bytes(int64_t n_pix, int32_t max_adc_values, int32_t n_paths) {
+  return record_layout(n_pix, max_adc_values, n_paths, nullptr, nullptr);
+}
+
+static ProbArgs prob_args(const LsimParams &p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths) {
+  ProbArgs a{};
   a.p = p;
   a.wfs = wfs;
   a.n_pix = n_pix;
@@ -906,65 +1137,81 @@ static ProbArgs prob_args(const LsimParams &p, const float *wfs, int64_t n_pix, 
   a.interval = p.fee_interval;
   a.z = (float)(1.0 / (double)p.reset_noise);
   a.thr = p.threshold;
+  return a;
+}
+
+static int check_prob(const LsimParams &p, int32_t n_t, int32_t n_paths) {
+  if (n_t < 3 || n_t > kProbMaxT) return set_error(LSIM_ERR_UNSUPPORTED, "probabilistic FEE: n_t must be in [3, 2048]");
+  if (n_paths < 1 || n_paths > kProbMaxPaths || n_paths > n_t - 1)
+    return set_error(LSIM_ERR_UNSUPPORTED, "probabilistic FEE: fee_paths_scaling must be in [1, min(32, n_t - 1)]");
+  if (!(p.reset_noise > 0.0f)) return set_error(LSIM_ERR_INVALID, "probabilistic FEE: RESET_NOISE_CHARGE must be > 0");
+  return LSIM_OK;
+}
+
+template <bool kDist>
+static int launch_prob(const ProbArgs &a, cudaStream_t st) {
+  const size_t smem = sizeof(float) * (kProbArrays * kProbMaxT + kProbExtraFloats);
+  if (cudaFuncSetAttribute(k_fee_prob<kDist>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return LSIM_ERR_CUDA;
+  const int64_t cap = prob_blocks();
+  k_fee_prob<kDist><<<(unsigned)(a.n_pix < cap ? a.n_pix : cap), kProbThreads, smem, st>>>(a);
+  return cudaGetLastError() == cudaSuccess ? LSIM_OK : LSIM_ERR_CUDA;
+}
+
+// record: null, or where the adjoint's record goes (fee_prob_record_bytes).
+// all_steps: the record serves cotangents on the log-probabilities too.
+static int run_fee_prob_impl(const LsimParams &p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
+                             float stop_threshold, float *log_prob, float *charge, float *e_tick, float *e_adc,
+                             float *lam, void *record, bool all_steps, void *ws, cudaStream_t st) {
+  int rc = check_prob(p, n_t, n_paths);
+  if (rc != LSIM_OK) return rc;
+  ProbArgs a = prob_args(p, wfs, n_pix, n_t, n_paths);
   a.log_stop = logf(stop_threshold);
   a.log_prob = log_prob;
   a.charge = charge;
   a.e_tick = e_tick;
   a.e_adc = e_adc;
   a.lam = lam;
-  a.step_active = static_cast<int32_t *>(ws);
-  a.state = nullptr;
-  a.state_top = nullptr;
-  return a;
-}
-
-static int run_fee_prob_impl(const LsimParams &p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
-                             float stop_threshold, float *log_prob, float *charge, float *e_tick, float *e_adc,
-                             float *lam, void *ws, float *state, int32_t *state_top, cudaStream_t st) {
-  if (n_t < 3 || n_t > kProbMaxT) return set_error(LSIM_ERR_UNSUPPORTED, "probabilistic FEE: n_t must be in [3, 2048]");
-  if (n_paths < 1 || n_paths > kProbMaxPaths || n_paths > n_t - 1)
-    return set_error(LSIM_ERR_UNSUPPORTED, "probabilistic FEE: fee_paths_scaling must be in [1, min(32, n_t - 1)]");
-  if (!(p.reset_noise > 0.0f)) return set_error(LSIM_ERR_INVALID, "probabilistic FEE: RESET_NOISE_CHARGE must be > 0");
-  ProbArgs a = prob_args(p, wfs, n_pix, n_t, n_paths, stop_threshold, log_prob, charge, e_tick, e_adc, lam, ws);
-  a.state = state;
-  a.state_top = state_top;
-  if (cudaMemsetAsync(a.step_active, 0, sizeof(int32_t) * p.max_adc_values, st) != cudaSuccess) return LSIM_ERR_CUDA;
+  a.all_steps = all_steps || charge != nullptr;
+  char *b = static_cast<char *>(ws);
+  a.step_active = reinterpret_cast<int32_t *>(b);
+  a.cache = reinterpret_cast<float *>(b + kFlagBytes);
+  if (record) {
+    ProbRecord r;
+    record_layout(n_pix, p.max_adc_values, n_paths, &r, static_cast<char *>(record));
+    a.step_active = r.step_active;
+    a.state = r.state;
+    a.state_top = r.top;
+    a.live = r.live;
+    a.n_run = r.n_run;
+    a.red = r.red;
+  }
+  a.work = work_counter(a.step_active);
+  if (cudaMemsetAsync(a.step_active, 0, kFlagBytes, st) != cudaSuccess) return LSIM_ERR_CUDA;
   if (n_pix == 0) return LSIM_OK;
-  const size_t smem = sizeof(float) * (kProbArrays * kProbMaxT + kProbExtraFloats);
-  if (cudaFuncSetAttribute(k_fee_prob, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return LSIM_ERR_CUDA;
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fee_prob, kProbThreads, smem);
-  const int64_t cap = (int64_t)device_sm_count() * (per_sm > 0 ? per_sm : 1);
-  const unsigned grid = (unsigned)(n_pix < cap ? n_pix : cap);
-  k_fee_prob<<<grid, kProbThreads, smem, st>>>(a);
+  rc = log_prob ? launch_prob<true>(a, st) : launch_prob<false>(a, st);
+  if (rc != LSIM_OK) return rc;
   if (log_prob || charge || lam)
     k_fee_prob_mask<<<(unsigned)device_sm_count() * 4, 256, 0, st>>>(a, p.max_adc_values);
-  return LSIM_OK;
+  return cudaGetLastError() == cudaSuccess ? LSIM_OK : LSIM_ERR_CUDA;
 }
 
-size_t fee_prob_vjp_workspace_bytes(int64_t n_pix, int32_t max_adc_values, int32_t n_paths) {
-  auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-  const size_t states = (size_t)(n_pix > 0 ? n_pix : 0) * (size_t)max_adc_values * (size_t)n_paths;
-  return fee_prob_workspace_bytes(max_adc_values) + al(sizeof(float) * 2 * states) + al(sizeof(int32_t) * states);
-}
-
-int run_fee_prob_vjp(const LsimParams &p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
-                     float stop_threshold, const float *g_log_prob, const float *g_charge, const float *g_e_tick,
-                     const float *g_e_adc, const float *g_lam, float *g_wfs, void *ws, cudaStream_t st) {
-  auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-  const size_t states = (size_t)n_pix * (size_t)p.max_adc_values * (size_t)n_paths;
-  char *b = static_cast<char *>(ws);
-  float *state = reinterpret_cast<float *>(b + fee_prob_workspace_bytes(p.max_adc_values));
-  int32_t *state_top = reinterpret_cast<int32_t *>(reinterpret_cast<char *>(state) + al(sizeof(float) * 2 * states));
-  // forward with the step states recorded (no outputs), then the reverse pass
-  int rc = run_fee_prob_impl(p, wfs, n_pix, n_t, n_paths, stop_threshold, nullptr, nullptr, nullptr, nullptr,
-                             nullptr, ws, state, state_top, st);
+// The reverse pass on a record.
+int run_fee_prob_vjp_recorded(const LsimParams &p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
+                              const void *record, const float *g_log_prob, const float *g_charge, const float *g_e_tick,
+                              const float *g_e_adc, const float *g_lam, float *g_wfs, cudaStream_t st) {
+  const int rc = check_prob(p, n_t, n_paths);
   if (rc != LSIM_OK || n_pix == 0) return rc;
-  ProbVjpArgs va;
-  va.f = prob_args(p, wfs, n_pix, n_t, n_paths, stop_threshold, nullptr, nullptr, nullptr, nullptr, nullptr, ws);
-  va.f.state = state;
-  va.f.state_top = state_top;
+  ProbRecord r;
+  record_layout(n_pix, p.max_adc_values, n_paths, &r, const_cast<char *>(static_cast<const char *>(record)));
+  ProbVjpArgs va{};
+  va.f = prob_args(p, wfs, n_pix, n_t, n_paths);
+  va.f.step_active = r.step_active;
+  va.f.state = r.state;
+  va.f.state_top = r.top;
+  va.f.live = r.live;
+  va.f.n_run = r.n_run;
+  va.f.red = r.red;
   va.g_log_prob = g_log_prob;
   va.g_charge = g_charge;
   va.g_e_tick = g_e_tick;
@@ -974,18 +1221,34 @@ int run_fee_prob_vjp(const LsimParams &p, const float *wfs, int64_t n_pix, int32
   const size_t smem = sizeof(float) * (kVjpArrays * kProbMaxT + 2 * (kProbThreads / 32) * kProbMaxPaths);
   if (cudaFuncSetAttribute(k_fee_prob_vjp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return LSIM_ERR_CUDA;
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fee_prob_vjp, kProbThreads, smem);
-  const int64_t cap = (int64_t)device_sm_count() * (per_sm > 0 ? per_sm : 1);
+  const int64_t cap = prob_blocks();
   k_fee_prob_vjp<<<(unsigned)(n_pix < cap ? n_pix : cap), kProbThreads, smem, st>>>(va);
   return cudaGetLastError() == cudaSuccess ? LSIM_OK : LSIM_ERR_CUDA;
 }
 
+size_t fee_prob_vjp_workspace_bytes(int64_t n_pix, int32_t max_adc_values, int32_t n_paths) {
+  return fee_prob_workspace_bytes(max_adc_values) + fee_prob_record_bytes(n_pix, max_adc_values, n_paths);
+}
+
+int run_fee_prob_vjp(const LsimParams &p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
+                     float stop_threshold, const float *g_log_prob, const float *g_charge, const float *g_e_tick,
+                     const float *g_e_adc, const float *g_lam, float *g_wfs, void *ws, cudaStream_t st) {
+  // the record, then the forward's workspace
+  char *record = static_cast<char *>(ws);
+  ws = record + fee_prob_record_bytes(n_pix, p.max_adc_values, n_paths);
+  // forward with the steps recorded, then the reverse pass
+  const int rc = run_fee_prob_impl(p, wfs, n_pix, n_t, n_paths, stop_threshold, nullptr, nullptr, nullptr, nullptr,
+                                   nullptr, record, g_log_prob != nullptr || g_charge != nullptr, ws, st);
+  if (rc != LSIM_OK) return rc;
+  return run_fee_prob_vjp_recorded(p, wfs, n_pix, n_t, n_paths, record, g_log_prob, g_charge, g_e_tick, g_e_adc,
+                                   g_lam, g_wfs, st);
+}
+
 int run_fee_prob(const LsimParams &p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
                  float stop_threshold, float *log_prob, float *charge, float *e_tick, float *e_adc, float *lam,
-                 void *ws, cudaStream_t st) {
-  return run_fee_prob_impl(p, wfs, n_pix, n_t, n_paths, stop_threshold, log_prob, charge, e_tick, e_adc, lam, ws,
-                           nullptr, nullptr, st);
+                 void *record, void *ws, cudaStream_t st) {
+  return run_fee_prob_impl(p, wfs, n_pix, n_t, n_paths, stop_threshold, log_prob, charge, e_tick, e_adc, lam, record,
+                           false, ws, st);
 }
 
 }  // namespace lsim

@@ -71,7 +71,11 @@ int run_pixel_coords(const LsimParams &p, const int32_t *unique_pixels, int64_t 
 size_t fee_prob_workspace_bytes(int32_t max_adc_values);
 int run_fee_prob(const LsimParams &p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
                  float stop_threshold, float *log_prob, float *charge, float *e_tick, float *e_adc, float *lam,
-                 void *ws, cudaStream_t st);
+                 void *record, void *ws, cudaStream_t st);
+size_t fee_prob_record_bytes(int64_t n_pix, int32_t max_adc_values, int32_t n_paths);
+int run_fee_prob_vjp_recorded(const LsimParams &p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
+                              const void *record, const float *g_log_prob, const float *g_charge, const float *g_e_tick,
+                              const float *g_e_adc, const float *g_lam, float *g_wfs, cudaStream_t st);
 
 // lsim_prob_loss.cu
 size_t prob_llhd_workspace_bytes(int64_t n_hits);

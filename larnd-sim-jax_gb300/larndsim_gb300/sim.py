@@ -352,7 +352,7 @@ def simulate_parametrized(params, tracks, fields, rngseed=0, offsets=None, norma
 
 # ---------------------------------------------------------------- probabilistic front end
 
-def _fee_prob(params, wfs, stop_threshold, distributions, reductions):
+def _fee_prob(params, wfs, stop_threshold, distributions, reductions, record=False):
     lib = _abi.load()
     w = torch.as_tensor(wfs).to(device=_device(), dtype=torch.float32).contiguous()
     if w.dim() != 2:
@@ -361,62 +361,67 @@ def _fee_prob(params, wfs, stop_threshold, distributions, reductions):
         raise ValueError("the probabilistic front end needs RESET_NOISE_CHARGE > 0 (its noise width)")
     P, T = w.shape
     H = int(params.MAX_ADC_VALUES)
+    K = int(params.fee_paths_scaling)
     lp = _abi.make_params(params)
     ws = torch.empty(lib.lsim_fee_prob_workspace_bytes(lp), dtype=torch.uint8, device=w.device)
     f = dict(dtype=torch.float32, device=w.device)
     log_prob = torch.empty((P, H, T - 1), **f) if distributions else None
     charge = torch.empty((P, H, T - 1), **f) if distributions else None
     red = [torch.empty((P, H), **f) for _ in range(3)] if reductions else [None] * 3
-    _abi.check(lib, lib.lsim_fee_prob(lp, _ptr(w), P, T, int(params.fee_paths_scaling), float(stop_threshold),
-                                      _ptr(log_prob), _ptr(charge), *(_ptr(r) for r in red), _ptr(ws),
-                                      ws.numel(), _stream()))
-    return log_prob, charge, red
+    outs = (_ptr(log_prob), _ptr(charge), *(_ptr(r) for r in red))
+    if not record:
+        _abi.check(lib, lib.lsim_fee_prob(lp, _ptr(w), P, T, K, float(stop_threshold), *outs, _ptr(ws), ws.numel(),
+                                          _stream()))
+        return log_prob, charge, red, None
+    rec = torch.empty(lib.lsim_fee_prob_record_bytes(lp, P, max(K, 1)), dtype=torch.uint8, device=w.device)
+    _abi.check(lib, lib.lsim_fee_prob_record(lp, _ptr(w), P, T, K, float(stop_threshold), *outs, _ptr(rec),
+                                             rec.numel(), _ptr(ws), ws.numel(), _stream()))
+    return log_prob, charge, red, rec
 
 
-def _fee_prob_vjp(params, wfs, stop_threshold, g_lp=None, g_ch=None, g_red=None):
+def _fee_prob_vjp(params, wfs, rec, g_lp=None, g_ch=None, g_red=None):
     lib = _abi.load()
     w = wfs.detach().to(dtype=torch.float32).contiguous()
     P, T = w.shape
     lp = _abi.make_params(params)
-    K = int(params.fee_paths_scaling)
-    ws = torch.empty(lib.lsim_fee_prob_vjp_workspace_bytes(lp, P, K), dtype=torch.uint8, device=w.device)
     g = torch.empty_like(w)
     c = lambda t: None if t is None else t.to(torch.float32).contiguous()   # noqa: E731
-    red = [None] * 3 if g_red is None else [c(t) for t in g_red]
+    g_red = [None] * 3 if g_red is None else [c(t) for t in g_red]
     g_lp, g_ch = c(g_lp), c(g_ch)
-    _abi.check(lib, lib.lsim_fee_prob_vjp(lp, _ptr(w), P, T, K, float(stop_threshold), _ptr(g_lp), _ptr(g_ch),
-                                          *(_ptr(r) for r in red), _ptr(g), _ptr(ws), ws.numel(), _stream()))
+    _abi.check(lib, lib.lsim_fee_prob_vjp_recorded(lp, _ptr(w), P, T, int(params.fee_paths_scaling), _ptr(rec),
+                                                   rec.numel(), _ptr(g_lp), _ptr(g_ch), *(_ptr(r) for r in g_red), _ptr(g),
+                                                   _stream()))
     return g
 
 
 class _FeeProbDistFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, wfs, params, stop_threshold):
-        log_prob, charge, _ = _fee_prob(params, wfs, stop_threshold, True, False)
-        ctx.save_for_backward(wfs)
-        ctx.params, ctx.stop = params, stop_threshold
+        log_prob, charge, _, rec = _fee_prob(params, wfs, stop_threshold, True, False, ctx.needs_input_grad[0])
+        ctx.save_for_backward(wfs, rec)
+        ctx.params = params
         return log_prob, charge
 
     @staticmethod
     def backward(ctx, g_lp, g_ch):
-        (wfs,) = ctx.saved_tensors
-        return _fee_prob_vjp(ctx.params, wfs, ctx.stop, g_lp=g_lp, g_ch=g_ch), None, None
+        wfs, rec = ctx.saved_tensors
+        return _fee_prob_vjp(ctx.params, wfs, rec, g_lp=g_lp, g_ch=g_ch), None, None
 
 
 class _FeeProbRedFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, wfs, params, stop_threshold):
-        _, _, (e_tick, e_adc, lam) = _fee_prob(params, wfs, stop_threshold, False, True)
-        ctx.save_for_backward(wfs)
-        ctx.params, ctx.stop = params, stop_threshold
+        _, _, (e_tick, e_adc, lam), rec = _fee_prob(params, wfs, stop_threshold, False, True, ctx.needs_input_grad[0])
+        ctx.save_for_backward(wfs, rec)
+        ctx.params = params
         return e_tick, e_adc, lam
 
     @staticmethod
     def backward(ctx, g_t, g_a, g_l):
-        (wfs,) = ctx.saved_tensors
+        wfs, rec = ctx.saved_tensors
         zero = lambda g: torch.zeros(wfs.shape[0], int(ctx.params.MAX_ADC_VALUES), device=wfs.device) \
             if g is None else g   # noqa: E731
-        return _fee_prob_vjp(ctx.params, wfs, ctx.stop, g_red=(zero(g_t), zero(g_a), zero(g_l))), None, None
+        return _fee_prob_vjp(ctx.params, wfs, rec, g_red=(zero(g_t), zero(g_a), zero(g_l))), None, None
 
 
 def _as_wfs(wfs):
