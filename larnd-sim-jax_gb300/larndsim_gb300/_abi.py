@@ -10,6 +10,7 @@ and rounding once, the way the reference's static parameters behave.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import threading
 from pathlib import Path
 
@@ -231,15 +232,24 @@ def field_map(fields, n_fields=None) -> LsimFieldMap:
     return fm
 
 
-def _f32(x) -> float:
-    return float(np.float32(x))
+# Values that a few numbers determine (not objects): the same for every call
+# with the same detector.
+@functools.lru_cache(maxsize=64)
+def _param_ticks(npt):
+    return tuple(consts.jax_linspace_f32(0, 5, npt).tolist())
+
+
+@functools.lru_cache(maxsize=64)
+def _tran_edges(nb, pitch, bins):
+    return tuple(consts.tran_diff_edges(nb, pitch, bins).tolist())
 
 
 def make_params(params, lut_shape=None) -> LsimParams:
     """Fill an LsimParams block from a Params object.
 
     ``lut_shape`` = (n_templates, nx, ny, nt) of the template bank (LUT
-    mode); omitted in parametrised mode.
+    mode); omitted in parametrised mode.  Expressions are evaluated in
+    float64 and rounded once, by the assignment to the float32 field.
     """
     lp = LsimParams()
     mode = getattr(params.recombination_mode, "value", params.recombination_mode)
@@ -247,41 +257,38 @@ def make_params(params, lut_shape=None) -> LsimParams:
         raise ValueError(f"Invalid recombination mode {params.recombination_mode}: "
                          "must be RecombinationMode.BOX, RecombinationMode.BIRKS, or RecombinationMode.ELLIPSOID")
     lp.recombination_mode = int(mode)
-    lp.Ab, lp.kb = _f32(params.Ab), _f32(params.kb)
-    lp.alpha, lp.beta = _f32(params.alpha), _f32(params.beta)
-    lp.r_inv2 = _f32(1.0 / params.R_param ** 2)
-    lp.erho = _f32(params.eField * params.lArDensity)
-    lp.mev_to_electrons = _f32(params.MeVToElectrons)
-    lp.vdrift = _f32(consts.get_vdrift(params))
-    lp.lifetime, lp.long_diff, lp.tran_diff = _f32(params.lifetime), _f32(params.long_diff), _f32(params.tran_diff)
-    lp.size_margin = _f32(params.size_margin)
-    lp.shift_x, lp.shift_y, lp.shift_z = _f32(params.shift_x), _f32(params.shift_y), _f32(params.shift_z)
+    lp.Ab, lp.kb = float(params.Ab), float(params.kb)
+    lp.alpha, lp.beta = float(params.alpha), float(params.beta)
+    lp.r_inv2 = float(1.0 / params.R_param ** 2)
+    lp.erho = float(params.eField * params.lArDensity)
+    lp.mev_to_electrons = float(params.MeVToElectrons)
+    lp.vdrift = float(consts.get_vdrift(params))
+    lp.lifetime, lp.long_diff, lp.tran_diff = float(params.lifetime), float(params.long_diff), float(params.tran_diff)
+    lp.size_margin = float(params.size_margin)
+    lp.shift_x, lp.shift_y, lp.shift_z = float(params.shift_x), float(params.shift_y), float(params.shift_z)
     b = np.asarray(params.tpc_borders, np.float32)
     if b.shape[0] > MAX_TPC or b.shape[1:] != (3, 2):
         raise ValueError(f"tpc_borders of shape {b.shape} not supported")
     lp.n_tpc = b.shape[0]
-    for i, v in enumerate(b.ravel()):
-        lp.tpc_borders[i] = float(v)
+    lp.tpc_borders[:b.size] = b.ravel().tolist()
     nb = int(params.nb_sampling_bins_per_pixel)
-    lp.pixel_pitch = _f32(params.pixel_pitch)
-    lp.half_pitch = _f32(params.pixel_pitch / 2)
-    lp.bin_width = _f32(params.pixel_pitch / nb)
+    lp.pixel_pitch = float(params.pixel_pitch)
+    lp.half_pitch = float(params.pixel_pitch / 2)
+    lp.bin_width = float(params.pixel_pitch / nb)
     lp.n_pixels_x, lp.n_pixels_y = int(params.n_pixels_x), int(params.n_pixels_y)
     lp.nb_bins_per_pixel = nb
     lp.n_tran_bins = int(params.nb_tran_diff_bins)
     lp.n_neighbors = int(params.number_pix_neighbors)
-    edges = consts.tran_diff_bin_edges(params)
-    for i, v in enumerate(edges[:8]):
-        lp.tran_edges[i] = float(v)
-    lp.t_sampling = _f32(params.t_sampling)
+    edges = _tran_edges(int(params.nb_tran_diff_bins), float(params.pixel_pitch), float(nb))[:8]
+    lp.tran_edges[:len(edges)] = edges
+    lp.t_sampling = float(params.t_sampling)
     lp.n_ticks = consts.n_ticks(params)
     lp.signal_length = int(params.signal_length)
     tmpl = np.asarray(params.long_diff_template, np.float32)
     if tmpl.shape[0] > MAX_TEMPLATES:
         raise ValueError(f"{tmpl.shape[0]} long-diffusion templates > {MAX_TEMPLATES}")
     lp.n_templates = tmpl.shape[0]
-    for i, v in enumerate(tmpl):
-        lp.long_diff_template[i] = float(v)
+    lp.long_diff_template[:tmpl.shape[0]] = tmpl.tolist()
     if lut_shape is not None:
         nt_, nx, ny, nt = (int(v) for v in lut_shape)
         if nt_ != tmpl.shape[0]:
@@ -291,15 +298,15 @@ def make_params(params, lut_shape=None) -> LsimParams:
             raise ValueError(f"a {nx}x{ny} LUT covers fewer than the {need} sub-pixel positions that "
                              f"number_pix_neighbors={params.number_pix_neighbors} reads")
         lp.lut_nx, lp.lut_ny, lp.lut_nt = nx, ny, nt
-    lp.threshold = _f32(params.DISCRIMINATION_THRESHOLD)
-    lp.gain = _f32(params.GAIN)
-    lp.v_pedestal = _f32(params.V_PEDESTAL)
-    lp.v_cm = _f32(params.V_CM)
-    lp.vref_minus_cm = _f32(params.V_REF - params.V_CM)
-    lp.adc_counts = _f32(params.ADC_COUNTS)
-    lp.reset_noise = _f32(params.RESET_NOISE_CHARGE)
-    lp.uncorr_noise = _f32(params.UNCORRELATED_NOISE_CHARGE)
-    lp.hit_prob_threshold = _f32(params.hit_prob_threshold)
+    lp.threshold = float(params.DISCRIMINATION_THRESHOLD)
+    lp.gain = float(params.GAIN)
+    lp.v_pedestal = float(params.V_PEDESTAL)
+    lp.v_cm = float(params.V_CM)
+    lp.vref_minus_cm = float(params.V_REF - params.V_CM)
+    lp.adc_counts = float(params.ADC_COUNTS)
+    lp.reset_noise = float(params.RESET_NOISE_CHARGE)
+    lp.uncorr_noise = float(params.UNCORRELATED_NOISE_CHARGE)
+    lp.hit_prob_threshold = float(params.hit_prob_threshold)
     lp.max_adc_values = int(params.MAX_ADC_VALUES)
     if not 1 <= lp.max_adc_values <= MAX_HITS:
         raise ValueError(f"MAX_ADC_VALUES {lp.max_adc_values} not in [1, {MAX_HITS}]")
@@ -309,11 +316,10 @@ def make_params(params, lut_shape=None) -> LsimParams:
     if npt > 64:
         raise ValueError("parametrised current window longer than 64 ticks")
     lp.param_nticks = npt
-    lp.param_dt = _f32(5.0 / (npt - 1))
-    for i, v in enumerate(consts.jax_linspace_f32(0, 5, npt)):
-        lp.param_ticks[i] = float(v)
-    lp.eField, lp.lArDensity = _f32(params.eField), _f32(params.lArDensity)
-    lp.dvdrift_deField = _f32(consts.get_vdrift_derivative(params))
+    lp.param_dt = float(5.0 / (npt - 1))
+    lp.param_ticks[:npt] = _param_ticks(npt)
+    lp.eField, lp.lArDensity = float(params.eField), float(params.lArDensity)
+    lp.dvdrift_deField = float(consts.get_vdrift_derivative(params))
     for i, v in enumerate(params.ELECTRON_MOBILITY_PARAMS):
         lp.mobility[i] = float(v)
     lp.mobility_temp = pow(params.temperature / 89, -1.5) / 1000

@@ -198,12 +198,16 @@ def fee_interval(params) -> int:
     return round((3 * params.CLOCK_CYCLE + params.ADC_HOLD_DELAY * params.CLOCK_CYCLE) / params.t_sampling)
 
 
-def tran_diff_bin_edges(params) -> np.ndarray:
-    """Sub-pixel bin edges of the 5x5 transverse-diffusion grid (sim_jax.py:398-403)."""
-    nb = params.nb_tran_diff_bins
+def tran_diff_edges(nb, pitch, bins_per_pixel) -> np.ndarray:
+    """Sub-pixel bin edges of the nb x nb transverse-diffusion grid (sim_jax.py:398-403)."""
     sym = (nb - 1) // 2
-    width = params.pixel_pitch / params.nb_sampling_bins_per_pixel
+    width = pitch / bins_per_pixel
     return jax_linspace_f32(-sym * width, (sym + 1) * width, nb + 1)
+
+
+def tran_diff_bin_edges(params) -> np.ndarray:
+    """tran_diff_edges of the parameters' grid."""
+    return tran_diff_edges(params.nb_tran_diff_bins, params.pixel_pitch, params.nb_sampling_bins_per_pixel)
 
 
 def load_detector_properties(params_cls, detprop_file, pixel_file):
