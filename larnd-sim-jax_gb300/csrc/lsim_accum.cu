@@ -715,53 +715,63 @@ constexpr int kMainBlocks = 256;     // reduction blocks over per-segment main-b
 constexpr int kTgtBlocks = 256;      // reduction blocks over target-only rows
 static_assert(kPixBlocks + kMainBlocks + kTgtBlocks <= kRedSlots, "reduction partials");
 
-// Fixed-order float64 sum of per-pixel (or per-warp) records [loss, 8
-// gradient terms]: block b reduces a contiguous chunk; the chunking depends
-// only on the record count (n_fixed, or the valid-pixel count when < 0).
-__global__ void k_reduce_records(const float *__restrict__ pix, int64_t n_fixed, const LsimCounts *counts,
-                                 double *partials) {
-  __shared__ double sh[kRedThreads];
-  const int64_t n = n_fixed >= 0 ? n_fixed : counts->n_valid;
-  const int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
-  const int64_t lo = blockIdx.x * chunk, hi = min(n, lo + chunk);
-  for (int q = 0; q <= LSIM_NPARAM; ++q) {
-    double s = 0.0;
-    for (int64_t i = lo + threadIdx.x; i < hi; i += kRedThreads) s += (double)pix[i * kPixRec + q];
-    sh[threadIdx.x] = s;
+// Sum over the block of nine values per thread, in the order of a halving
+// tree over the threads; thread 0 gets it.
+template <int N>
+__device__ __forceinline__ void block_tree_sum(double (&v)[N], double (*sh)[kRedThreads / 2]) {
+#pragma unroll
+  for (int o = kRedThreads / 2; o >= kWarp; o >>= 1) {
+    if (threadIdx.x >= o && threadIdx.x < 2 * o)
+#pragma unroll
+      for (int q = 0; q < N; ++q) sh[q][threadIdx.x - o] = v[q];
     __syncthreads();
-    for (int o = kRedThreads / 2; o > 0; o >>= 1) {
-      if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) partials[(size_t)blockIdx.x * 16 + q] = sh[0];
+    if (threadIdx.x < o)
+#pragma unroll
+      for (int q = 0; q < N; ++q) v[q] += sh[q][threadIdx.x];
     __syncthreads();
   }
+  if (threadIdx.x < kWarp)
+#pragma unroll
+    for (int o = kWarp / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < N; ++q) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
 }
 
-// Row of the loss target with the pixel id of each valid pixel (both lists
-// are sorted), or -1.
-__global__ void k_target_index(AccumArgs a) {
-  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (r >= a.w.counts->n_valid) return;
-  const int32_t pid = slot_pid(a.p, a.g, a.w.pix_slot[r]);
-  int64_t lo = 0, hi = a.n_tgt;
-  while (lo < hi) {
-    const int64_t mid = (lo + hi) >> 1;
-    if (a.tgt_pids[mid] < pid) lo = mid + 1; else hi = mid;
+// Fixed-order float64 sum of per-pixel or per-segment records [loss, 8
+// gradient terms]: block b of `blocks` reduces a contiguous chunk; the
+// chunking depends only on the record count.  One pass over the records (nine
+// passes with a tree each took 30 us a launch even for a small event).
+__device__ __forceinline__ void reduce_records(const float *__restrict__ rec, int64_t n, int b, int blocks,
+                                               double *partials, double (*sh)[kRedThreads / 2]) {
+  const int64_t chunk = (n + blocks - 1) / blocks;
+  const int64_t lo = b * chunk, hi = min(n, lo + chunk);
+  double v[1 + LSIM_NPARAM];
+#pragma unroll
+  for (int q = 0; q <= LSIM_NPARAM; ++q) v[q] = 0.0;
+  for (int64_t i = lo + threadIdx.x; i < hi; i += kRedThreads) {
+    const float4 *r = reinterpret_cast<const float4 *>(rec + i * kPixRec);
+    const float4 x = r[0], y = r[1], z = r[2];
+    const float f[1 + LSIM_NPARAM] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w, z.x};
+#pragma unroll
+    for (int q = 0; q <= LSIM_NPARAM; ++q) v[q] += (double)f[q];
   }
-  a.w.tgt_index[r] = (lo < a.n_tgt && a.tgt_pids[lo] == pid) ? (int32_t)lo : -1;
+  block_tree_sum(v, sh);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int q = 0; q <= LSIM_NPARAM; ++q) partials[(size_t)b * 16 + q] = v[q];
 }
+static_assert(kPixRec == 12, "records are three float4");
 
-// Loss terms of target pixels that the prediction does not have.
-__global__ void k_target_only(AccumArgs a, double *partials) {
-  __shared__ double sh[kRedThreads];
+// Loss terms of target pixels that the prediction does not have (block b).
+__device__ __forceinline__ void target_only(const AccumArgs &a, int b, double *partials,
+                                            double (*sh)[kRedThreads / 2]) {
   const LsimParams &p = a.p;
   const int H = p.max_adc_values;
   const float adc0 = digitize(p, 0.f);
   const int n_valid = a.w.counts->n_valid;
-  const int64_t chunk = (a.n_tgt + gridDim.x - 1) / gridDim.x;
-  const int64_t lo = blockIdx.x * chunk, hi = min(a.n_tgt, lo + chunk);
-  double acc = 0.0;
+  const int64_t chunk = (a.n_tgt + kTgtBlocks - 1) / kTgtBlocks;
+  const int64_t lo = b * chunk, hi = min(a.n_tgt, lo + chunk);
+  double acc[1] = {0.0};
   for (int64_t t = lo + threadIdx.x; t < hi; t += kRedThreads) {
     const int32_t pid = a.tgt_pids[t];
     int l = 0, h2 = n_valid;
@@ -773,16 +783,25 @@ __global__ void k_target_only(AccumArgs a, double *partials) {
     if (!present && pid >= 0)
       for (int h = 0; h < H; ++h) {
         const float d = adc0 - a.tgt_adc[t * H + h];
-        acc += (double)(d * d);
+        acc[0] += (double)(d * d);
       }
   }
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  for (int o = kRedThreads / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) partials[(size_t)blockIdx.x * 16] = sh[0];
+  block_tree_sum(acc, sh);
+  if (threadIdx.x == 0) partials[(size_t)b * 16] = acc[0];
+}
+
+// All partial sums of a gradient call: the blocks of the pixel records, of
+// the main-bin records and (tgt_blocks of them) of the target's own pixels.
+__global__ void __launch_bounds__(kRedThreads) k_grad_partials(AccumArgs a) {
+  __shared__ double sh[1 + LSIM_NPARAM][kRedThreads / 2];
+  double *partials = a.w.red_partials;
+  const int b = blockIdx.x;
+  if (b < kPixBlocks)
+    reduce_records(a.w.pix_out, a.w.counts->n_valid, b, kPixBlocks, partials, sh);
+  else if (b < kPixBlocks + kMainBlocks)
+    reduce_records(a.w.main_out, a.n_rows, b - kPixBlocks, kMainBlocks, partials + (size_t)kPixBlocks * 16, sh);
+  else
+    target_only(a, b - kPixBlocks - kMainBlocks, partials + (size_t)(kPixBlocks + kMainBlocks) * 16, sh);
 }
 
 // One block per output (0: loss, 1..8: gradient): fixed-order float64 sum
@@ -816,9 +835,7 @@ __global__ void k_grad_finalize(const double *partials, int n_rec_blocks, const 
 // (contributions) are listed so that the persistent kernel starts with them.
 constexpr int kHeavyPixel = 2048;
 
-__global__ void k_heavy_pixels(Grid g, Workspace w) {
-  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (r >= w.counts->n_valid) return;
+__device__ __forceinline__ void mark_heavy(const Grid &g, const Workspace &w, int64_t r) {
   const int64_t slot = w.pix_slot[r];
   int cost = 0;
   for (int dy = -g.h; dy <= g.h; ++dy)
@@ -828,11 +845,37 @@ __global__ void k_heavy_pixels(Grid g, Workspace w) {
   if (heavy) w.heavy[atomicAdd(&w.counts->n_heavy, 1)] = (int32_t)r;
 }
 
-static int run_heavy_pixels(const AccumArgs &a, cudaStream_t st) {
-  if (cudaMemsetAsync(&a.w.counts->n_heavy, 0, sizeof(int32_t), st) != cudaSuccess) return LSIM_ERR_CUDA;
-  if (a.n_rows <= 0) return LSIM_OK;
-  k_heavy_pixels<<<(unsigned)((a.n_rows + 255) / 256), 256, 0, st>>>(a.g, a.w);
-  return cudaGetLastError() == cudaSuccess ? LSIM_OK : LSIM_ERR_CUDA;
+// Row of the loss target with the pixel id of valid pixel r (both lists are
+// sorted), or -1.
+__device__ __forceinline__ void find_target(const AccumArgs &a, int64_t r) {
+  const int32_t pid = slot_pid(a.p, a.g, a.w.pix_slot[r]);
+  int64_t lo = 0, hi = a.n_tgt;
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) >> 1;
+    if (a.tgt_pids[mid] < pid) lo = mid + 1; else hi = mid;
+  }
+  a.w.tgt_index[r] = (lo < a.n_tgt && a.tgt_pids[lo] == pid) ? (int32_t)lo : -1;
+}
+
+// A call's counters (a workspace may serve several calls).
+__global__ void k_pass_reset(Workspace w, bool records) {
+  if (threadIdx.x == 0) {
+    w.counts->work = 0;
+    w.counts->n_heavy = 0;
+    if (records) w.counts->n_main_rec = w.counts->n_main_seg = 0;
+  }
+  if (records)
+    for (int i = threadIdx.x; i < kMaxTemplates; i += blockDim.x) w.tidx_hist[i] = 0;
+}
+
+// What a call needs before its large kernels, one thread per row: the
+// template-order counts (records), the heavy pixels, the target rows.
+__global__ void k_pass_prepare(AccumArgs a, bool records, bool targets) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (records) main_order_count(a.w, a.n_rows, i);   // whole warps: it votes
+  if (i >= a.w.counts->n_valid) return;
+  mark_heavy(a.g, a.w, i);
+  if (targets) find_target(a, i);
 }
 
 // ---------------------------------------------------------------- launch
@@ -873,7 +916,6 @@ static int launch_mode(const AccumArgs &a0, cudaStream_t st) {
   if (rc != LSIM_OK) return rc;
   AccumArgs a = a0;
   a.warp_smem = (int)warp_smem_bytes<MODE>(a0.p);
-  if (cudaMemsetAsync(&a.w.counts->work, 0, sizeof(int32_t), st) != cudaSuccess) return LSIM_ERR_CUDA;
   cudaEvent_t ev0, ev1;
   kernel_events(&ev0, &ev1);
   if (ev0 && cudaEventRecord(ev0, st) != cudaSuccess) return LSIM_ERR_CUDA;
@@ -898,44 +940,31 @@ int run_accum(AccumMode mode, const AccumArgs &a, cudaStream_t st) {
     return LSIM_ERR_UNSUPPORTED;
   // the stored-waveform adjoint reuses the records (and their template
   // order) of the simulate_wfs pass that wrote the waveforms
-  int rc = mode == kModeGradStored ? LSIM_OK : run_main_records(a, st);
-  if (rc == LSIM_OK) rc = run_heavy_pixels(a, st);
+  const bool records = mode != kModeGradStored;
+  const bool targets = (mode == kModeGrad || mode == kModeGradStored) && !a.g_adc && a.n_tgt > 0;
+  if (records && a.n_rows > 0 && a.p.n_templates > kMaxTemplates) return LSIM_ERR_UNSUPPORTED;
+  k_pass_reset<<<1, 256, 0, st>>>(a.w, records);
+  if (a.n_rows > 0)
+    k_pass_prepare<<<(unsigned)((a.n_rows + 255) / 256), 256, 0, st>>>(a, records, targets);
+  int rc = records ? run_main_records(a, st) : LSIM_OK;
+  if (cudaGetLastError() != cudaSuccess) return LSIM_ERR_CUDA;
   if (rc != LSIM_OK) return rc;
   switch (mode) {
     case kModeWfs: return launch_mode<kModeWfs>(a, st);
     case kModeAdc: return launch_mode<kModeAdc>(a, st);
-    case kModeGrad:
-      if (!a.g_adc && a.n_tgt > 0 && a.n_rows > 0) {
-        k_target_index<<<(unsigned)((a.n_rows + 255) / 256), 256, 0, st>>>(a);
-        if (cudaGetLastError() != cudaSuccess) return LSIM_ERR_CUDA;
-      }
-      rc = launch_mode<kModeGrad>(a, st);
-      return rc != LSIM_OK ? rc : run_main_adjoint(a, st);
-    case kModeVjpWfs:
-      rc = launch_mode<kModeVjpWfs>(a, st);
-      return rc != LSIM_OK ? rc : run_main_adjoint(a, st);
-    case kModeGradStored:
-      if (!a.g_adc && a.n_tgt > 0 && a.n_rows > 0) {
-        k_target_index<<<(unsigned)((a.n_rows + 255) / 256), 256, 0, st>>>(a);
-        if (cudaGetLastError() != cudaSuccess) return LSIM_ERR_CUDA;
-      }
-      rc = launch_mode<kModeGradStored>(a, st);
-      return rc != LSIM_OK ? rc : run_main_adjoint(a, st);
+    case kModeGrad: rc = launch_mode<kModeGrad>(a, st); break;
+    case kModeVjpWfs: rc = launch_mode<kModeVjpWfs>(a, st); break;
+    case kModeGradStored: rc = launch_mode<kModeGradStored>(a, st); break;
+    default: return LSIM_ERR_INVALID;
   }
-  return LSIM_ERR_INVALID;
+  return rc != LSIM_OK ? rc : run_main_adjoint(a, st);
 }
 
 int run_grad_finalize(const AccumArgs &a, float *loss_out, float *grad_out, cudaStream_t st) {
   double *rec_partials = a.w.red_partials;
   double *tgt_partials = a.w.red_partials + (size_t)(kPixBlocks + kMainBlocks) * 16;
-  k_reduce_records<<<kPixBlocks, kRedThreads, 0, st>>>(a.w.pix_out, -1, a.w.counts, rec_partials);
-  k_reduce_records<<<kMainBlocks, kRedThreads, 0, st>>>(a.w.main_out, a.n_rows, a.w.counts,
-                                                        rec_partials + (size_t)kPixBlocks * 16);
-  int tb = 0;
-  if (!a.g_adc && a.n_tgt > 0) {
-    tb = kTgtBlocks;
-    k_target_only<<<tb, kRedThreads, 0, st>>>(a, tgt_partials);
-  }
+  const int tb = !a.g_adc && a.n_tgt > 0 ? kTgtBlocks : 0;
+  k_grad_partials<<<kPixBlocks + kMainBlocks + tb, kRedThreads, 0, st>>>(a);
   k_grad_finalize<<<1 + LSIM_NPARAM, kRedThreads, 0, st>>>(rec_partials, kPixBlocks + kMainBlocks, tgt_partials, tb,
                                                          loss_out, grad_out);
   return cudaGetLastError() == cudaSuccess ? LSIM_OK : LSIM_ERR_CUDA;

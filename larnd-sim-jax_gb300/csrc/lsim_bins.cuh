@@ -80,4 +80,25 @@ __device__ __forceinline__ float cum_terms(const float *row, int cath, int Nt, i
   return vs - (v0 * (1.f - frac) + v1 * frac);
 }
 
+// Whether a segment has main-bin records (n_e != 0 and a grid slot), and its
+// template index.
+__device__ __forceinline__ bool main_active(const Workspace &w, int64_t s, int64_t n_rows, int *bin) {
+  if (s >= n_rows) return false;
+  const SegFwd &f = w.segf[s];
+  *bin = f.tidx;
+  return f.ne != 0.f && w.key[s] >= 0;
+}
+
+// Counts segment s under its template index (warp-aggregated atomics: one
+// per distinct index per warp; called by whole warps).
+__device__ __forceinline__ void main_order_count(const Workspace &w, int64_t n_rows, int64_t s) {
+  int bin = 0;
+  const bool act = main_active(w, s, n_rows, &bin);
+  const unsigned am = __ballot_sync(0xffffffffu, act);
+  if (act) {
+    const unsigned peers = __match_any_sync(am, bin);
+    if ((threadIdx.x % kWarp) == __ffs(peers) - 1) atomicAdd(&w.tidx_hist[bin], __popc(peers));
+  }
+}
+
 }  // namespace lsim

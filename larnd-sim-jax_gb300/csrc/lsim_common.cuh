@@ -175,9 +175,9 @@ inline Workspace carve_workspace(void *base, const LsimParams &p, int64_t n_rows
   size_t o_segp = take(sizeof(SegPar) * (size_t)n_rows);
   size_t o_key = take(4 * (size_t)n_rows);
   size_t o_pid = take(4 * (size_t)n_rows);
-  size_t o_cnt = take(4 * (size_t)g.G);
-  size_t o_off = take(4 * (size_t)g.G);
+  size_t o_cnt = take(4 * (size_t)g.G);   // zeroed together with the cursors behind it
   size_t o_cur = take(4 * (size_t)g.G);
+  size_t o_off = take(4 * (size_t)g.G);
   size_t o_list = take(4 * (size_t)n_rows);
   size_t o_pixs = take(4 * (size_t)n_rows);
   size_t o_em1 = take(4 * (size_t)n_rows);

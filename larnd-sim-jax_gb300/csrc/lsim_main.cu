@@ -111,27 +111,9 @@ static void main_shape(int *blocks, int *warps) {
 
 // ---------------------------------------------------------------- order
 
-// Segments with main-bin records (n_e != 0 and a grid slot), grouped by
-// template index with a counting sort (the order inside a group is
-// arbitrary).  Warp-aggregated atomics: one per distinct index per warp.
-__device__ __forceinline__ bool main_active(const Workspace &w, int64_t s, int64_t n_rows, int *bin) {
-  if (s >= n_rows) return false;
-  const SegFwd &f = w.segf[s];
-  *bin = f.tidx;
-  return f.ne != 0.f && w.key[s] >= 0;
-}
-
-__global__ void k_main_order_count(Workspace w, int64_t n_rows) {
-  const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  int bin = 0;
-  const bool act = main_active(w, s, n_rows, &bin);
-  const unsigned am = __ballot_sync(0xffffffffu, act);
-  if (act) {
-    const unsigned peers = __match_any_sync(am, bin);
-    if ((threadIdx.x % kWarp) == __ffs(peers) - 1) atomicAdd(&w.tidx_hist[bin], __popc(peers));
-  }
-}
-
+// Segments with main-bin records, grouped by template index with a counting
+// sort (the order inside a group is arbitrary); the counts are made by
+// k_pass_prepare (main_order_count).
 __global__ void k_main_order_scan(Workspace w) {
   __shared__ int sh[kMaxTemplates];
   const int t = threadIdx.x;
@@ -325,12 +307,8 @@ __global__ void __launch_bounds__(kMainBlockWarps * kWarp, 24 / kMainBlockWarps)
 }
 
 int run_main_records(const AccumArgs &a, cudaStream_t st) {
-  if (cudaMemsetAsync(&a.w.counts->n_main_rec, 0, 2 * sizeof(int32_t), st) != cudaSuccess) return LSIM_ERR_CUDA;
   if (a.n_rows <= 0) return LSIM_OK;
-  if (a.p.n_templates > kMaxTemplates) return LSIM_ERR_UNSUPPORTED;
-  if (cudaMemsetAsync(a.w.tidx_hist, 0, sizeof(int32_t) * kMaxTemplates, st) != cudaSuccess) return LSIM_ERR_CUDA;
   const unsigned nb = (unsigned)((a.n_rows + 255) / 256);
-  k_main_order_count<<<nb, 256, 0, st>>>(a.w, a.n_rows);
   k_main_order_scan<<<1, kMaxTemplates, 0, st>>>(a.w);
   k_main_order_scatter<<<nb, 256, 0, st>>>(a.w, a.n_rows);
   int blocks, warps;

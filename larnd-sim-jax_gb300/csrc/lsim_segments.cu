@@ -662,7 +662,6 @@ int run_pixel_map(const LsimParams &p, const Workspace &w0, const Grid &g, int64
     k_scan_final<<<(unsigned)nscan, kScanThreads, 0, st>>>(w.cnt, g.G, g, w.scan_blocks, w.off, w.pix_slot,
                                                           w.em1_slot);
   }
-  if (cudaMemsetAsync(w.cursor, 0, 4 * (size_t)g.G, st) != cudaSuccess) return LSIM_ERR_CUDA;
   if (n_rows > 0) k_scatter<<<(unsigned)((n_rows + 255) / 256), 256, 0, st>>>(w.key, n_rows, w.off, w.cursor, w.seg_list);
   if (g.G > 0) {
     k_sort_slots<<<(unsigned)((g.G + 255) / 256), 256, 0, st>>>(w.cnt, w.off, g.G, w.seg_list, w.big_slots,
@@ -679,7 +678,9 @@ int run_stage1(bool param_mode, const LsimParams &p, const LsimFieldMap &f, cons
   Grid g = make_grid(p, n_events);
   k_reset_counts<<<1, 32, 0, st>>>(w.counts);
   if (theta_dev) k_theta_derive<<<1, 32, 0, st>>>(p, theta_dev, w.theta_derived);
-  if (cudaMemsetAsync(w.cnt, 0, 4 * (size_t)g.G, st) != cudaSuccess) return LSIM_ERR_CUDA;
+  // slot counts and scatter cursors
+  if (cudaMemsetAsync(w.cnt, 0, (size_t)((char *)(w.cursor + g.G) - (char *)w.cnt), st) != cudaSuccess)
+    return LSIM_ERR_CUDA;
   if (n_rows > 0) {
     unsigned nb = (unsigned)((n_rows + 127) / 128);
     if (param_mode)
