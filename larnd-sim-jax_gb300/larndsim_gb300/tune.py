@@ -28,7 +28,7 @@ class LsimTuning(C.Structure):
 
 FIELDS = ("pixel_blocks_per_sm", "main_blocks", "main_block_warps")
 DEFAULT_CANDIDATES = tuple(
-    dict(zip(FIELDS, v)) for v in itertools.product((0, 4, 3), (512, 1024, 2048), (8, 4)))
+    dict(zip(FIELDS, v)) for v in itertools.product((0, 4, 3), (0, 1024), (0, 8)))   # 0: the library's default
 _cache: dict = {}
 
 
