@@ -252,7 +252,7 @@ constexpr float kWeakRise = 1.4f, kWeakMost = -190.0f;
 //   whose dist term is above kProbFar;
 // * a pixel whose paths have all become improbable beyond kProbDead stops.
 // Bound by instruction issue in the special functions.  Values and gradient of
-// 1500 dense rows: 42.4 -> 10.1 ms; distributions of 1000 rows: 8.8 -> 5.2 ms.
+// 1500 dense rows: 42.4 -> 6.5 ms (10.1 before the adjoint below); distributions of 1000 rows: 8.8 -> 5.2 ms.
 template <bool kDist>
 __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob(ProbArgs a) {
   extern __shared__ __align__(16) float sm[];
@@ -755,35 +755,39 @@ __device__ __forceinline__ float dlog_ndtr_f(float x, float lx) {
   return expf((-0.5f * x * x - 0.918938533204672742f) - lx);
 }
 
-// log_diff_ndtr value and partials d/da, d/db (la = log_ndtr(a), dla its derivative)
-__device__ __forceinline__ float ldn_grad(float a, float b, float la, float lb, float dla, float dlb, float term_m1,
-                                          float &ga, float &gb) {
-  float lts, dlts_du = 0.f;
-  const bool sel = a > b;
-  if (sel) {
-    const float u = lb - la;
-    const float neg = -expm1f(u);
-    const float y = (neg - 1e-30f) * 1e10f;
-    const float ns = 1e-30f + softplus_f(y) / 1e10f;
-    const float lt = logf(ns);
-    lts = -100.0f + ((lt + 100.0f) * 10.0f) / 10.0f;
-    // softplus' = sigmoid; d neg / du = -exp(u); the second clamp is the identity there
-    dlts_du = (1.0f / ns) * sigmoid_f(y) * (-expf(u));
-  } else {
-    lts = term_m1;
+// log_diff_ndtr and its partials d/da, d/db (la = log_ndtr(a), lb = log_ndtr(b))
+struct LogDiff {
+  float lp, w, out;       // log term, gate, value
+  float u, y, ns;         // of the log term where a > b
+  __device__ __forceinline__ LogDiff(float a, float b, float la, float lb, float term_m1) {
+    u = y = ns = 0.f;
+    float lts = term_m1;
+    if (a > b) {
+      u = lb - la;
+      const float neg = -expm1f(u);
+      y = (neg - 1e-30f) * 1e10f;
+      ns = 1e-30f + softplus_f(y) / 1e10f;
+      const float lt = logf(ns);
+      lts = -100.0f + ((lt + 100.0f) * 10.0f) / 10.0f;
+    }
+    lp = la + lts;
+    w = sigmoid_f((a - b) * 1000.0f);
+    out = w * lp + (1.0f - w) * kProbFloor;
   }
-  const float lp = la + lts;
-  const float w = sigmoid_f((a - b) * 1000.0f);
-  const float out = w * lp + (1.0f - w) * kProbFloor;
-  const float gw = (lp - kProbFloor) * w * (1.0f - w) * 1000.0f;   // through the gate
-  ga = w * (dla - dlts_du * dla) + gw;
-  gb = w * (dlts_du * dlb) - gw;
-  if (!sel) {
-    ga = w * dla + gw;
-    gb = -gw;
+  __device__ __forceinline__ void partials(float a, float b, float la, float lb, float &ga, float &gb) const {
+    const float dla = dlog_ndtr_f(a, la);
+    const float gw = (lp - kProbFloor) * w * (1.0f - w) * 1000.0f;   // through the gate
+    if (a > b) {
+      // softplus' = sigmoid; d neg / du = -exp(u); the second clamp is the identity there
+      const float dlts_du = (1.0f / ns) * sigmoid_f(y) * (-expf(u));
+      ga = w * (dla - dlts_du * dla) + gw;
+      gb = w * (dlts_du * dlog_ndtr_f(b, lb)) - gw;
+    } else {
+      ga = w * dla + gw;
+      gb = -gw;
+    }
   }
-  return out;
-}
+};
 
 struct ProbVjpArgs {
   ProbArgs f;                  // the forward's arguments (its record, step_active and reductions read)
@@ -805,15 +809,28 @@ struct ProbVjpArgs {
 //
 // Few classes of a step have a cotangent at all: those of the K selected
 // ticks and those whose probability is not 0 (the forward's record says
-// which), about 5 % of the ticks.  A step lists them, and the 16 warps take
-// one class at a time, lane k for path k: the log-sum-exps, the partials'
-// sums over the paths and the class's ticks are all within a warp.  (A thread
-// per class, walking the K paths, left one or two warps of a block at work
-// and recomputed every class's log-sum-exps: 1500 rows took 16.1 ms.)
+// which), about 10 % of the ticks.  A step lists them and takes as many at a
+// time as there are threads for their (class, path) pairs: a thread evaluates
+// the special functions of one pair, with paths that repeat a likelier path's
+// charge left out (the first step has one path).  The weights exp(x - max) of
+// a class's log-sum-exp stay unnormalised until its sums are formed, so the
+// sums over the paths are a thread per (class, quantity) adding what the
+// pairs left in shared memory, without shuffles; four lanes per class spread
+// them to its ticks.
+// Bound by instruction issue in the special functions, of which each lane
+// should have one to evaluate: adjoint of 1500 dense rows 16.1 ms with a
+// thread per class walking the K paths, 5.6 ms with a warp per class (15.5 of
+// 32 lanes had a path) and the rows dealt in turn, 2.6 ms so.
 constexpr int kVjpSpan = 16;
-constexpr int kVjpArrays = 12;   // q, running max, 5 accumulators, dist cotangents, scratch, class, representative,
-                                 // list of live classes; the esperance and the soft-where weight are recomputed from
-                                 // q, so two blocks fit on an SM
+constexpr int kVjpArrays = 9;      // q, running max, 5 accumulators, dist cotangents, scratch; the esperance and the
+                                   // soft-where weight are recomputed from q, so two blocks fit on an SM
+constexpr int kVjpShorts = 3;      // class, representative, list of live classes (16 bits: ticks < kProbMaxT)
+// what the pairs leave for their class: hit and dist terms; the hit weight and five partials times it, the dist weight
+// and two partials times it (a class's sums then replace its first pair's); the hit terms' maximum
+enum PairValue { kPairHit, kPairDist, kPairSums, kPairDistSums = kPairSums + 6, kPairMax = kPairDistSums + 3, kPairValues };
+constexpr int kPairStride = kProbThreads + 1;   // quantities of one pair in different banks
+constexpr int kTickLanes = 4;                   // lanes that share a class's ticks
+static_assert(kProbMaxT <= 65536, "16-bit tick indices");
 
 __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va) {
   extern __shared__ __align__(16) float sm[];
@@ -821,13 +838,14 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
   float *qs = sm, *cm = qs + kProbMaxT;
   float *Aq0 = cm + kProbMaxT, *Aqs = Aq0 + kProbMaxT, *Am0 = Aqs + kProbMaxT, *Am1 = Am0 + kProbMaxT;
   float *Aesp = Am1 + kProbMaxT, *Gd = Aesp + kProbMaxT, *tmp = Gd + kProbMaxT;
-  int *cls = reinterpret_cast<int *>(tmp + kProbMaxT), *rep = cls + kProbMaxT, *list = rep + kProbMaxT;
-  float *part = reinterpret_cast<float *>(list + kProbMaxT);   // [warps][2][kProbMaxPaths]
+  float *pair = tmp + kProbMaxT;                               // [kPairValues][kPairStride]
+  uint16_t *cls = reinterpret_cast<uint16_t *>(pair + kPairValues * kPairStride);
+  uint16_t *rep = cls + kProbMaxT, *list = rep + kProbMaxT;
   __shared__ float red[kProbThreads / 32];
   __shared__ float pc[kProbMaxPaths], plp[kProbMaxPaths], glp_n[kProbMaxPaths], gc_n[kProbMaxPaths];
-  __shared__ int pskip[kProbMaxPaths], ptop[kProbMaxPaths];
-  __shared__ int counts[kProbTicks][kProbThreads / 32];
-  __shared__ int n_exec, n_cls;
+  __shared__ int ptop[kProbMaxPaths], act[kProbMaxPaths];
+  __shared__ int counts[kProbTicks * (kProbThreads / 32)];
+  __shared__ int n_exec, n_cls, n_act;
 
   const LsimParams &p = a.p;
   const int T = a.T, K = a.K, H = p.max_adc_values, tid = threadIdx.x;
@@ -876,8 +894,8 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
     block_scan_row<kScanSum>(tmp, T - 1, red);   // integer counts, exact in float32
     for (int t = tid; t < T - 1; t += kProbThreads) {
       const int u = (int)tmp[t] - 1;
-      cls[t] = u;
-      if (t == 0 || (int)tmp[t - 1] != u + 1) rep[u] = t;
+      cls[t] = (uint16_t)u;
+      if (t == 0 || (int)tmp[t - 1] != u + 1) rep[u] = (uint16_t)t;
       if (t == T - 2) n_cls = u + 1;
     }
     if (tid < K) {
@@ -886,7 +904,7 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
     }
     __syncthreads();
     const int U = n_cls;
-    if (tid == 0) rep[U] = T - 1;     // end of the last class
+    if (tid == 0) rep[U] = (uint16_t)(T - 1);     // end of the last class
 
     for (int h = min(n_exec, a.n_run[pix]) - 1; h >= 0; --h) {
       const int64_t o = pix * H + h;
@@ -899,20 +917,37 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
       }
       for (int t = tid; t < T; t += kProbThreads) Gd[t] = tmp[t] = 0.f;
       __syncthreads();
-      if (tid < K) {
-        int sk = 0;
+      if (wid == 0) {
+        // the paths that count, in order (a path whose charge repeats that of one more than 110 log units likelier
+        // adds nothing)
+        bool on = lane < K;
         for (int j = 0; j < K; ++j)
-          if (j != tid && pc[j] == pc[tid] && plp[j] > plp[tid] + 110.0f) sk = 1;
-        pskip[tid] = sk;
-        if (glp_n[tid] != 0.f) tmp[cls[ptop[tid]]] = 1.f;   // the class has a dist cotangent
+          if (lane < K && j != lane && pc[j] == pc[lane] && plp[j] > plp[lane] + 110.0f) on = false;
+        const unsigned bal = __ballot_sync(0xffffffffu, on);
+        if (on) act[__popc(bal & ((1u << lane) - 1u))] = lane;
+        if (lane == 0) n_act = __popc(bal);
+        if (lane < K && glp_n[lane] != 0.f) tmp[cls[ptop[lane]]] = 1.f;   // the class has a dist cotangent
       }
-      if (tid == 0) {
-        // the next step's state cotangents: new lp_j = dist[top_j], new c_j = q[best_j]
-        for (int j = 0; j < K; ++j) {
-          const int tt = ptop[j];
-          Gd[tt] += glp_n[j];
-          Aq0[min(shifted(tt) + 1, T - 1)] += gc_n[j];
-        }
+      if (wid == 1) {
+        // the next step's state cotangents: new lp_j = dist[top_j], new c_j = q[best_j].  The first lane of those with
+        // the same tick adds them all, in order
+        auto add_to = [&](float *dst, int t, float v) {
+          const bool on = lane < K;
+          float sum = on ? dst[t] : 0.f;
+          bool first = on;
+          for (int j = 0; j < K; ++j) {
+            const int tj = __shfl_sync(0xffffffffu, t, j);
+            const float vj = __shfl_sync(0xffffffffu, v, j);
+            if (tj == t) {
+              sum += vj;
+              if (j < lane) first = false;
+            }
+          }
+          if (first) dst[t] = sum;
+        };
+        const int tt = lane < K ? ptop[lane] : 0;
+        add_to(Gd, tt, lane < K ? glp_n[lane] : 0.f);
+        add_to(Aq0, min(shifted(tt) + 1, T - 1), lane < K ? gc_n[lane] : 0.f);
       }
       if (va.g_charge)
         for (int t = tid; t < T - 1; t += kProbThreads) Aesp[t] += va.g_charge[o * (int64_t)(T - 1) + t];
@@ -931,17 +966,30 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
             for (int tt = t; tt < rep[u + 1] && !live; ++tt) live = va.g_log_prob[o * (int64_t)(T - 1) + tt] != 0.f;
         }
         live_bits[i] = __ballot_sync(0xffffffffu, live);
-        if (lane == 0) counts[i][wid] = __popc(live_bits[i]);
+        if (lane == 0) counts[i * (kProbThreads / 32) + wid] = __popc(live_bits[i]);
       }
       __syncthreads();
-      int n_live = 0;
+      int n_live;
+      {
+        static_assert(kProbTicks * (kProbThreads / 32) == 64, "two counts a lane");
+        const int c0 = counts[2 * lane], c1 = counts[2 * lane + 1];
+        int incl = c0 + c1;
 #pragma unroll
-      for (int i = 0; i < kProbTicks; ++i)
-        for (int w2 = 0; w2 < kProbThreads / 32; ++w2) {
-          if (w2 == wid && (live_bits[i] >> lane) & 1u)
-            list[n_live + __popc(live_bits[i] & ((1u << lane) - 1u))] = tid + i * kProbThreads;
-          n_live += counts[i][w2];
+        for (int o2 = 1; o2 < 32; o2 <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, incl, o2);
+          if (lane >= o2) incl += y;
         }
+        n_live = __shfl_sync(0xffffffffu, incl, 31);
+#pragma unroll
+        for (int i = 0; i < kProbTicks; ++i) {
+          const int at = i * (kProbThreads / 32) + wid;      // entry of the prefix sums
+          const int ex = __shfl_sync(0xffffffffu, incl - c0 - c1, at >> 1);
+          const int first = __shfl_sync(0xffffffffu, c0, at >> 1);
+          if ((live_bits[i] >> lane) & 1u)
+            list[ex + (at & 1 ? first : 0) + __popc(live_bits[i] & ((1u << lane) - 1u))] =
+                (uint16_t)(tid + i * kProbThreads);
+        }
+      }
       __syncthreads();
       // the reductions' cotangents, common to the step's ticks
       float gl = 0.f, gt = 0.f, ga = 0.f, den = 1.f;
@@ -954,92 +1002,159 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
         // the lambda cotangent also reaches ET and EA through the denominator
         gl = va.g_lam[o] + on * (-(gt * ET + ga * EA) / den);
       }
-      const bool path = lane < K && !pskip[lane < K ? lane : 0];
-      const float c = lane < K ? pc[lane] : 0.f, lp = lane < K ? plp[lane] : 0.f;
-      float glp = 0.f, gc = 0.f;      // lane k: path k's cotangents
-      for (int e = wid; e < n_live; e += kProbThreads / 32) {
-        const int u = list[e], t = rep[u], nt = rep[u + 1] - t;
-        const int sidx = shifted(t);
-        // ---- lane k: path k's values and partials at the class
-        const float zm0 = ((cm[t] - c) - thr) * z, zm1 = ((cm[t + 1] - c) - thr) * z;
-        const float LM0 = log_ndtr_f(zm0), LM1 = log_ndtr_f(zm1);
-        float g_m1, g_m0;
-        const float lg = ldn_grad(zm1, zm0, LM1, LM0, dlog_ndtr_f(zm1, LM1), dlog_ndtr_f(zm0, LM0), term_m1, g_m1,
-                                  g_m0);
-        const float zq0 = ((qs[t] - c) - thr) * z, zqs = ((qs[sidx] - c) - thr) * z;
-        const float LQ0 = log_ndtr_f(zq0), LQs = log_ndtr_f(zqs);
-        float g_qs, g_q0;
-        const float lep = ldn_grad(zqs, zq0, LQs, LQ0, dlog_ndtr_f(zqs, LQs), dlog_ndtr_f(zq0, LQ0), term_m1, g_qs,
-                                   g_q0);
-        const float le1 = fminf(lep, lg);
-        const float le2 = kProbFloor + softplus_f(le1 - kProbFloor);
-        const float wt = sw_at(esp_at(t));
-        const float le = wt * le2 + (1.0f - wt) * kProbFloor;
-        // ---- hit and dist log-sum-exps
-        auto lse = [&](float x) {
-          float m = path ? x : -INFINITY;
-#pragma unroll
-          for (int s2 = 16; s2 > 0; s2 >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s2));
-          return logf(warp_sum(path ? expf(x - m) : 0.f)) + m;
+      auto at = [&](int what, int i) -> float & { return pair[what * kPairStride + i]; };
+      const int na = n_act, per_round = kProbThreads / na;   // classes per round of pairs
+      const int my = tid / na;                                // this thread's class in a round
+      float glp = 0.f, gc = 0.f;                              // cotangents of its path act[tid - my na]
+      for (int e0 = 0; e0 < n_live; e0 += per_round) {
+        const int n_round = min(per_round, n_live - e0);
+        const bool on = my < n_round;
+        // ---- a thread per (class, path): values and partials at the class
+        float xh = 0.f, xd = 0.f, v_q0 = 0.f, v_qs = 0.f, r = 0.f, v_m0 = 0.f, v_m1 = 0.f, v_e = 0.f;
+        bool dist = false;     // the class has a dist cotangent
+        if (on) {
+          const int u = list[e0 + my], k = act[tid - my * na], t = rep[u], sidx = shifted(t);
+          dist = tmp[u] != 0.f;
+          const float c = pc[k], lp = plp[k];
+          const float zm0 = ((cm[t] - c) - thr) * z, zm1 = ((cm[t + 1] - c) - thr) * z;
+          const float LM0 = log_ndtr_f(zm0), LM1 = log_ndtr_f(zm1);
+          const LogDiff dm(zm1, zm0, LM1, LM0, term_m1);
+          const float zq0 = ((qs[t] - c) - thr) * z, zqs = ((qs[sidx] - c) - thr) * z;
+          const float LQ0 = log_ndtr_f(zq0), LQs = log_ndtr_f(zqs);
+          const LogDiff dq(zqs, zq0, LQs, LQ0, term_m1);
+          const float lg = dm.out, lep = dq.out;
+          // the cotangent of the smaller term only (both at a tie)
+          float g_m1 = 0.f, g_m0 = 0.f, g_qs = 0.f, g_q0 = 0.f;
+          if (dist || !(lep < lg)) dm.partials(zm1, zm0, LM1, LM0, g_m1, g_m0);
+          if (!(lep > lg)) dq.partials(zqs, zq0, LQs, LQ0, g_qs, g_q0);
+          const float le1 = fminf(lep, lg);
+          const float le2 = kProbFloor + softplus_f(le1 - kProbFloor);
+          const float wt = sw_at(esp_at(t));
+          const float le = wt * le2 + (1.0f - wt) * kProbFloor;
+          // per unit hit cotangent: le = w le2 + (1 - w)(-1000), w = sigmoid((esp - thr) 10)
+          const float gl1 = wt * sigmoid_f(le1 - kProbFloor);
+          const float s_lep = lep < lg ? 1.f : (lep == lg ? 0.5f : 0.f);
+          xh = le + lp;
+          xd = lg + lp;
+          v_q0 = gl1 * s_lep * g_q0 * z;
+          v_qs = gl1 * s_lep * g_qs * z;
+          r = gl1 * (1.f - s_lep);
+          v_m0 = g_m0 * z;
+          v_m1 = g_m1 * z;
+          v_e = (le2 - kProbFloor) * wt * (1.0f - wt) * 10.0f;
+          at(kPairHit, tid) = xh;
+          at(kPairDist, tid) = xd;
+        }
+        __syncthreads();
+        // ---- weights of the log-sum-exps and the partials times them
+        auto highest = [&](const float *x) {
+          float m = -INFINITY;
+          for (int j = 0; j < na; ++j) m = fmaxf(m, x[j]);
+          return m;
         };
-        const float vh = lse(le + lp), vd = lse(lg + lp);
-        // ---- the class's ticks, lane j for its tick j
-        float gh = 0.f, gd = 0.f;
-        if (lane < nt) {
-          const int tt = t + lane;
-          if (va.g_log_prob) gh = va.g_log_prob[o * (int64_t)(T - 1) + tt];
-          gd = Gd[tt];
-          if (va.g_lam) {
-            const float pr = expf(vh), et = esp_at(tt);
-            gh += (gl + gt * (float)tt / den + ga * digitize(p, et) / den) * pr;
-            Aesp[tt] += digitize_vjp(p, et, ga * pr / den);
+        float wh = 0.f, wd = 0.f, gh_c = 0.f, gd_c = 0.f;   // weights; charge partials times them
+        if (on) {
+          const float m = highest(&at(kPairHit, my * na));
+          wh = expf(xh - m);
+          const float p0 = wh * v_q0, ps = wh * v_qs, pm0 = wh * (r * v_m0), pm1 = wh * (r * v_m1);
+          gh_c = p0 + ps + pm0 + pm1;
+          at(kPairSums, tid) = wh;
+          at(kPairSums + 1, tid) = p0;
+          at(kPairSums + 2, tid) = ps;
+          at(kPairSums + 3, tid) = pm0;
+          at(kPairSums + 4, tid) = pm1;
+          at(kPairSums + 5, tid) = wh * v_e;
+          if (tid == my * na) at(kPairMax, tid) = m;
+          if (dist) {
+            wd = expf(xd - highest(&at(kPairDist, my * na)));
+            const float d0 = wd * v_m0, d1 = wd * v_m1;
+            gd_c = d0 + d1;
+            at(kPairDistSums, tid) = wd;
+            at(kPairDistSums + 1, tid) = d0;
+            at(kPairDistSums + 2, tid) = d1;
           }
         }
-        const bool any_h = __any_sync(0xffffffffu, gh != 0.f), any_d = __any_sync(0xffffffffu, gd != 0.f);
-        const float Hs = warp_sum(gh), Ds = warp_sum(gd);
-        // d(hit log-sum-exp)/d(le + lp) and d(dist log-sum-exp)/d(lg + lp)
-        const float al = any_h && path ? expf((le + lp) - vh) : 0.f;
-        const float be = any_d && path ? expf((lg + lp) - vd) : 0.f;
-        // per unit hit cotangent: le = w le2 + (1 - w)(-1000), w = sigmoid((esp - thr) 10)
-        const float gl1 = al * wt * sigmoid_f(le1 - kProbFloor);
-        const float s_lep = lep < lg ? 1.f : (lep == lg ? 0.5f : 0.f);
-        const float hl = gl1 * s_lep, hg = gl1 * (1.f - s_lep);
-        float co[7];
-        co[0] = hl * g_q0 * z;
-        co[1] = hl * g_qs * z;
-        co[2] = hg * g_m0 * z;
-        co[3] = be * g_m0 * z;
-        co[4] = hg * g_m1 * z;
-        co[5] = be * g_m1 * z;
-        co[6] = al * (le2 - kProbFloor) * wt * (1.0f - wt) * 10.0f;
-        if (path) {
-          glp += al * Hs + be * Ds;
-          gc -= (Hs * (hl * (g_q0 + g_qs) + hg * (g_m0 + g_m1)) + Ds * be * (g_m0 + g_m1)) * z;
+        __syncthreads();
+        // ---- a thread per (class, quantity): the sums over the paths
+        constexpr int kSums = kPairMax - kPairSums;
+        for (int i = tid; i < n_round * kSums; i += kProbThreads) {
+          const int e = i / kSums, what = kPairSums + i % kSums;
+          if (what >= kPairDistSums && tmp[list[e0 + e]] == 0.f) continue;
+          float *x = &at(what, e * na), sum = 0.f;
+          for (int j = 0; j < na; ++j) sum += x[j];
+          x[0] = sum;
         }
+        __syncthreads();
+        // ---- kTickLanes lanes per class: its ticks
+        for (int i = tid; (i & ~31) < n_round * kTickLanes; i += kProbThreads) {
+          const int e = i / kTickLanes;
+          const bool mine = e < n_round;
+          float Hs = 0.f, Ds = 0.f, inv = 0.f, inv_d = 0.f;
+          if (mine) {
+            const int u = list[e0 + e], f = e * na;
+            const bool with_d = tmp[u] != 0.f;
+            const float S = at(kPairSums, f), pr = expf(logf(S) + at(kPairMax, f));
+            inv = 1.0f / S;
+            inv_d = with_d ? 1.0f / at(kPairDistSums, f) : 0.f;
+            for (int tt = rep[u] + i % kTickLanes; tt < rep[u + 1]; tt += kTickLanes) {
+              float gh = 0.f, add_e = 0.f;
+              const float gd = Gd[tt];
+              if (va.g_log_prob) gh = va.g_log_prob[o * (int64_t)(T - 1) + tt];
+              if (va.g_lam) {
+                const float et = esp_at(tt);
+                gh += (gl + gt * (float)tt / den + ga * digitize(p, et) / den) * pr;
+                add_e = digitize_vjp(p, et, ga * pr / den);
+              }
+              Hs += gh;
+              Ds += gd;
+              const float n = gh * inv, nd = gd * inv_d;
+              Aq0[tt] += n * at(kPairSums + 1, f);
+              Aqs[tt] += n * at(kPairSums + 2, f);
+              Aesp[tt] += add_e + n * at(kPairSums + 5, f);
+              float m0 = n * at(kPairSums + 3, f), m1 = n * at(kPairSums + 4, f);
+              if (with_d) {
+                m0 += nd * at(kPairDistSums + 1, f);
+                m1 += nd * at(kPairDistSums + 2, f);
+              }
+              Am0[tt] += m0;
+              Am1[tt] += m1;
+            }
+          }
 #pragma unroll
-        for (int j = 0; j < 7; ++j) co[j] = warp_sum(path ? co[j] : 0.f);
-        if (lane < nt) {
-          const int tt = t + lane;
-          Aq0[tt] += gh * co[0];
-          Aqs[tt] += gh * co[1];
-          Am0[tt] += gh * co[2] + gd * co[3];
-          Am1[tt] += gh * co[4] + gd * co[5];
-          Aesp[tt] += gh * co[6];
+          for (int s2 = kTickLanes / 2; s2 > 0; s2 >>= 1) {
+            Hs += __shfl_xor_sync(0xffffffffu, Hs, s2);
+            Ds += __shfl_xor_sync(0xffffffffu, Ds, s2);
+          }
+          if (mine && i % kTickLanes == 0) {
+            at(kPairMax, e * na) = Hs * inv;
+            at(kPairDistSums, e * na) = Ds * inv_d;
+          }
+        }
+        __syncthreads();
+        // ---- the pair's path (the next round writes these two values only after its first barrier)
+        if (on) {
+          const float n = at(kPairMax, my * na);
+          glp += wh * n;
+          gc -= gh_c * n;
+          if (dist) {
+            const float nd = at(kPairDistSums, my * na);
+            glp += wd * nd;
+            gc -= gd_c * nd;
+          }
         }
       }
-      if (lane < K) {
-        part[(wid * 2) * kProbMaxPaths + lane] = glp;
-        part[(wid * 2 + 1) * kProbMaxPaths + lane] = gc;
-      }
-      __syncthreads();
-      if (tid < K) {
-        float s1 = 0.f, s2 = 0.f;
-        for (int w2 = 0; w2 < kProbThreads / 32; ++w2) {
-          s1 += part[(w2 * 2) * kProbMaxPaths + tid];
-          s2 += part[(w2 * 2 + 1) * kProbMaxPaths + tid];
+      if (h > 0) {
+        // cotangent of this step's input state = the previous step's output state
+        at(kPairHit, tid) = glp;
+        at(kPairDist, tid) = gc;
+        if (tid < K) glp_n[tid] = gc_n[tid] = 0.f;    // paths that do not count have none
+        __syncthreads();
+        const int n_used = min(per_round, n_live);
+        if (wid < 2 && lane < na) {
+          float sum = 0.f;
+          for (int j = 0; j < n_used; ++j) sum += at(wid == 0 ? kPairHit : kPairDist, j * na + lane);
+          (wid == 0 ? glp_n : gc_n)[act[lane]] = sum;
         }
-        glp_n[tid] = s1;   // cotangent of this step's input state = the previous step's output state
-        gc_n[tid] = s2;
       }
       __syncthreads();
     }
@@ -1053,8 +1168,11 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
       float g = Aq0[t];
       const bool start = t == 0 || cm[t] != cm[t - 1];
       if (start) {
-        int e = t;
-        while (e + 1 < T && cm[e + 1] == cm[t]) ++e;
+        int e = t, hi = T;        // last tick of the run: cm does not fall (and is never NaN)
+        while (hi - e > 1) {
+          const int mid = (e + hi) >> 1;
+          if (cm[mid] == cm[t]) e = mid; else hi = mid;
+        }
         g += tmp[e] - (t > 0 ? tmp[t - 1] : 0.f);
       }
       // shifted-tick role q[s_t] (s_t = min(t + interval + 1, T - 1)), with the esperance terms
@@ -1218,10 +1336,15 @@ int run_fee_prob_vjp_recorded(const LsimParams &p, const float *wfs, int64_t n_p
   va.g_e_adc = g_e_adc;
   va.g_lam = g_lam;
   va.g_wfs = g_wfs;
-  const size_t smem = sizeof(float) * (kVjpArrays * kProbMaxT + 2 * (kProbThreads / 32) * kProbMaxPaths);
+  const size_t smem = sizeof(float) * (kVjpArrays * kProbMaxT + kPairValues * kPairStride) +
+                      sizeof(uint16_t) * kVjpShorts * kProbMaxT;
   if (cudaFuncSetAttribute(k_fee_prob_vjp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return LSIM_ERR_CUDA;
-  const int64_t cap = prob_blocks();
+  // a block per pixel: pixels differ several times in cost, and blocks start as
+  // others end (the record is only read, so it has no place for a counter).
+  // 1500 rows, with a warp per class: 5.6 ms with the rows dealt in turn to the
+  // resident blocks, 4.8 ms so
+  constexpr int64_t cap = 1 << 30;
   k_fee_prob_vjp<<<(unsigned)(n_pix < cap ? n_pix : cap), kProbThreads, smem, st>>>(va);
   return cudaGetLastError() == cudaSuccess ? LSIM_OK : LSIM_ERR_CUDA;
 }
