@@ -83,6 +83,7 @@ __device__ __forceinline__ int list_dy(int cd) { return ((cd >> 4) & 15) - 4; }
 // and the slot's offset (dx, dy) from the pixel.
 __device__ __forceinline__ bool neigh_lookup(const ListSmem &ls, int g, int *pos, int *dx, int *dy) {
   int lo = 0, hi = ls.n;                 // last entry with pre_n <= g
+#pragma unroll 1
   while (hi - lo > 1) {
     int mid = (lo + hi) >> 1;
     if (ls.pre_n[mid] <= g) lo = mid; else hi = mid;
@@ -264,6 +265,31 @@ struct Theta {
   float v[LSIM_NPARAM];
 };
 
+// The sums of neigh_vjp_one over a window that crosses the edge of the
+// waveform: sum v gA, sum v gB, and gA, gB of the lane's first sample.  (Edge
+// windows are few and kept out of line here and below: the kernel's
+// instructions do not fit in the cache otherwise.)
+static __device__ __noinline__ float4 neigh_vjp_edge(float v0, float v1, float v2, float v3, float v4, int cb, int L,
+                                                     int NT, const float *grow, int lane) {
+  static_assert(kChunks == 5, "neigh_vjp_edge takes the five chunks by value");
+  const float v[kChunks] = {v0, v1, v2, v3, v4};
+  float sA = 0.f, sB = 0.f, gA0 = 0.f, gB0 = 0.f;
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) {
+    const int idx = c * kWarp + lane;
+    if (idx <= L) {
+      const int c1 = cb + idx;
+      const int lo = idx == 0 ? 1 : 2, hi = idx == 0 ? NT - 2 : NT - 1;
+      const float gA = (c1 >= lo && c1 <= hi) ? grow[c1] : 0.f;
+      const float gB = (c1 + 1 >= lo && c1 + 1 <= hi) ? grow[c1 + 1] : 0.f;
+      sA = fmaf(v[c], gA, sA);
+      sB = fmaf(v[c], gB, sB);
+      if (c == 0) { gA0 = gA; gB0 = gB; }
+    }
+  }
+  return make_float4(sA, sB, gA0, gB0);
+}
+
 // Adjoint of one neighbour contribution (descriptor d) given its padded
 // template-0 samples v[c] = w0[row][32c + lane] (sample idx - 1 of the
 // window, idx = 32c + lane): sample k lands on columns cb + k + 1 (x frac)
@@ -290,19 +316,11 @@ __device__ __forceinline__ void neigh_vjp_one(const NDesc &d, const float v[kChu
     sA = sAB.x;
     sB = sAB.y;
   } else {
-#pragma unroll
-    for (int c = 0; c < kChunks; ++c) {
-      const int idx = c * kWarp + lane;
-      if (idx <= L) {
-        const int c1 = cb + idx;
-        const int lo = idx == 0 ? 1 : 2, hi = idx == 0 ? NT - 2 : NT - 1;
-        const float gA = (c1 >= lo && c1 <= hi) ? grow[c1] : 0.f;
-        const float gB = (c1 + 1 >= lo && c1 + 1 <= hi) ? grow[c1 + 1] : 0.f;
-        sA = fmaf(v[c], gA, sA);
-        sB = fmaf(v[c], gB, sB);
-        if (c == 0) { gA0 = gA; gB0 = gB; }
-      }
-    }
+    const float4 e = neigh_vjp_edge(v[0], v[1], v[2], v[3], v[4], cb, L, NT, grow, lane);
+    sA = e.x;
+    sB = e.y;
+    gA0 = e.z;
+    gB0 = e.w;
   }
   float acc_ne = sA * f + sB * f1, acc_fr = sA - sB;
   if (lane == 0) {
@@ -359,48 +377,53 @@ template <bool GRAD, typename F>
 __device__ __forceinline__ void main_batches(const LsimParams &p, const Workspace &w, const ListSmem &ls, NBatch &nb,
                                              int lane, F &&flush) {
   constexpr int nbp = kBinsPerPixel;
-  int m = 0;
-  for (int e = 0; e < ls.n; ++e) {
-    const int cd = ls.cd[e];
-    const int dx = list_dx(cd), dy = list_dy(cd);
-    if (dx < -1 || dx > 1 || dy < -1 || dy > 1) continue;
-    const int o = ls.off[e], c = list_count(cd);
-    for (int j0 = 0; j0 < c; j0 += kWarp) {
-      int s = 0, slot = 0;
-      bool hit = false;
-      if (j0 + lane < c) {
-        s = __ldg(w.seg_list + o + j0 + lane);
-        const SegFwd &f = w.segf[s];
-        int lx, hx, ly, hy;
-        axis_range(__ldg(&f.bx), nbp, &lx, &hx);
-        axis_range(__ldg(&f.by), nbp, &ly, &hy);
-        hit = __ldg(&f.ne) != 0.f && lx <= dx && dx <= hx && ly <= dy && dy <= hy;
-        slot = (dx - lx) * 2 + (dy - ly);
-      }
-      const unsigned bal = __ballot_sync(0xffffffffu, hit);
-      const int nh = __popc(bal);
-      if (m + nh > kWarp) {
-        flush(m);
-        m = 0;
-      }
-      if (hit) {
-        const int pos = m + __popc(bal & ((1u << lane) - 1u));
-        const SegFwd &f = w.segf[s];
-        const int rec = s * kRecPerSeg + slot;
-        const int cb = p.lut_nt - p.signal_length - __ldg(&f.cath) - 1;
-        const float frac = __ldg(&f.frac);
-        NDesc d;
-        d.w = make_float4(1.f - frac, frac, GRAD ? w.mrec[(size_t)rec * kRecFloats + kRecDl] : 0.f,
-                          pack_window(0, cb, window_interior(cb, p.signal_length, p.n_ticks)));
-        d.g0 = make_float4(GRAD ? __ldg(&w.sega[s].dt0) / p.t_sampling : 0.f, __int_as_float(rec), 0.f, 0.f);
-        d.g1 = make_float4(0.f, 0.f, 0.f, 0.f);
-        nb.d[pos] = d;
-      }
-      m += nh;
-      __syncwarp();
+  int m = 0;                           // descriptors in the batch
+  int e = -1, c = 0, j0 = 0, o = 0;    // slot, its segments, the next candidate
+  int dx = 0, dy = 0;
+  for (;;) {                           // (one call of flush: its code is large)
+    while (j0 >= c && ++e < ls.n) {
+      const int cd = ls.cd[e];
+      dx = list_dx(cd), dy = list_dy(cd);
+      o = ls.off[e];
+      c = dx < -1 || dx > 1 || dy < -1 || dy > 1 ? 0 : list_count(cd);
+      j0 = 0;
     }
+    const bool last = e >= ls.n;
+    int s = 0, slot = 0;
+    bool hit = false;
+    if (!last && j0 + lane < c) {
+      s = __ldg(w.seg_list + o + j0 + lane);
+      const SegFwd &f = w.segf[s];
+      int lx, hx, ly, hy;
+      axis_range(__ldg(&f.bx), nbp, &lx, &hx);
+      axis_range(__ldg(&f.by), nbp, &ly, &hy);
+      hit = __ldg(&f.ne) != 0.f && lx <= dx && dx <= hx && ly <= dy && dy <= hy;
+      slot = (dx - lx) * 2 + (dy - ly);
+    }
+    j0 += kWarp;
+    const unsigned bal = __ballot_sync(0xffffffffu, hit);
+    const int nh = __popc(bal);
+    if (m > 0 && (last || m + nh > kWarp)) {
+      flush(m);
+      m = 0;
+    }
+    if (last) break;
+    if (hit) {
+      const int pos = m + __popc(bal & ((1u << lane) - 1u));
+      const SegFwd &f = w.segf[s];
+      const int rec = s * kRecPerSeg + slot;
+      const int cb = p.lut_nt - p.signal_length - __ldg(&f.cath) - 1;
+      const float frac = __ldg(&f.frac);
+      NDesc d;
+      d.w = make_float4(1.f - frac, frac, GRAD ? w.mrec[(size_t)rec * kRecFloats + kRecDl] : 0.f,
+                        pack_window(0, cb, window_interior(cb, p.signal_length, p.n_ticks)));
+      d.g0 = make_float4(GRAD ? __ldg(&w.sega[s].dt0) / p.t_sampling : 0.f, __int_as_float(rec), 0.f, 0.f);
+      d.g1 = make_float4(0.f, 0.f, 0.f, 0.f);
+      nb.d[pos] = d;
+    }
+    m += nh;
+    __syncwarp();
   }
-  if (m) flush(m);
 }
 
 // Forward: add m batched records (window samples k = -1 .. 158 stored at
@@ -438,6 +461,31 @@ __device__ __forceinline__ void main_rec_forward(const LsimParams &p, const floa
   __syncwarp();
 }
 
+// main_rec_backward's record whose window crosses the edge of the waveform:
+// the fraction's cotangent and lane 0's boundary correction's.
+static __device__ __noinline__ float2 main_rec_vjp_edge(float u0, float u1, float u2, float u3, float u4, float *rec,
+                                                        float f, float f1, int cb, int L, int NT, const float *grow,
+                                                        int lane) {
+  static_assert(kChunks == 5, "main_rec_vjp_edge takes the five chunks by value");
+  const float u[kChunks] = {u0, u1, u2, u3, u4};
+  float dfr = 0.f, dcorr = 0.f;
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) {
+    const int idx = lane + c * kWarp;
+    if (idx <= L) {
+      const int c1 = cb + idx;
+      const int lo = idx == 0 ? 1 : 2, hi = idx == 0 ? NT - 2 : NT - 1;
+      const float gA = (c1 >= lo && c1 <= hi) ? grow[c1] : 0.f;
+      const float gB = (c1 + 1 >= lo && c1 + 1 <= hi) ? grow[c1 + 1] : 0.f;
+      const float du = gA * f + gB * f1;
+      rec[idx] = du;
+      dfr += u[c] * (gA - gB);
+      if (idx == 0) dcorr = du;
+    }
+  }
+  return make_float2(dfr, dcorr);
+}
+
 // Adjoint of m batched records given the waveform cotangent grow[col]:
 // each record is replaced by the cotangent of its samples (rec[0]: the
 // boundary correction, rec[1 + k]: V[k]); the sub-tick-fraction part goes
@@ -464,27 +512,23 @@ __device__ __forceinline__ void main_rec_backward(const LsimParams &p, float *mr
     const int pk = __float_as_int(d.w.w);
     const int cb = pack_cb(pk);
     const float f1 = d.w.x, f = d.w.y;
-    const bool interior = !(pk & kPackEdge);
     float dfr = 0.f, dcorr = 0.f;
+    if (!(pk & kPackEdge)) {
 #pragma unroll
-    for (int c = 0; c < kChunks; ++c) {
-      const int idx = lane + c * kWarp;     // sample idx - 1 lands on columns cb + idx (x frac), cb + idx + 1
-      if (idx <= L) {
-        const int c1 = cb + idx;
-        float gA, gB;
-        if (interior) {
-          gA = grow[c1];
-          gB = grow[c1 + 1];
-        } else {
-          const int lo = idx == 0 ? 1 : 2, hi = idx == 0 ? NT - 2 : NT - 1;
-          gA = (c1 >= lo && c1 <= hi) ? grow[c1] : 0.f;
-          gB = (c1 + 1 >= lo && c1 + 1 <= hi) ? grow[c1 + 1] : 0.f;
+      for (int c = 0; c < kChunks; ++c) {
+        const int idx = lane + c * kWarp;     // sample idx - 1 lands on columns cb + idx (x frac), cb + idx + 1
+        if (idx <= L) {
+          const float gA = grow[cb + idx], gB = grow[cb + idx + 1];
+          const float du = gA * f + gB * f1;
+          rec[idx] = du;
+          dfr += u[c] * (gA - gB);
+          if (idx == 0) dcorr = du;
         }
-        const float du = gA * f + gB * f1;
-        rec[idx] = du;
-        dfr += u[c] * (gA - gB);
-        if (idx == 0) dcorr = du;
       }
+    } else {
+      const float2 e = main_rec_vjp_edge(u[0], u[1], u[2], u[3], u[4], rec, f, f1, cb, L, NT, grow, lane);
+      dfr = e.x;
+      dcorr = e.y;
     }
     if (lane == 0) dfr += dcorr * d.w.z;
     th.v[2] = fmaf(dfr, d.g0.x, th.v[2]);
@@ -572,7 +616,14 @@ __device__ __forceinline__ int32_t slot_pid(const LsimParams &p, const Grid &g, 
 // while at most 1 in kHeavyFractionInv pixels is heavy.
 constexpr int kHeavyFractionInv = 8;
 
-template <int MODE>
+// The gradient modes hold a pixel's whole path, and their 20 warps per SM are
+// in different phases of it, so what bounds them besides the shared-memory
+// row updates is the instruction cache: rarely taken code is out of line,
+// loops over few elements are not unrolled, each large body has one call, and
+// runs without noise draws are compiled without (NOISE).  64-event gradient
+// step: this kernel 14.1 -> 11.5 ms with 126 -> 94 KB of instructions, at the
+// same registers and the same bits; one event of 5000 segments 258 -> 247 us.
+template <int MODE, bool NOISE>
 __global__ void __launch_bounds__(kAccWarps * kWarp, 5) k_lut_pixels(AccumArgs a) {
   // kModeVjpWfs: the cotangent row comes from memory (no forward, no front end)
   constexpr bool VJP = MODE == kModeVjpWfs;
@@ -596,7 +647,7 @@ __global__ void __launch_bounds__(kAccWarps * kWarp, 5) k_lut_pixels(AccumArgs a
   // shared segments and LUT rows, together in time
   const int n_heavy0 = a.w.counts->n_heavy;
   const int n_heavy = n_heavy0 * kHeavyFractionInv > n_valid ? 0 : n_heavy0;
-  const bool early_exit = (a.normals == nullptr) && p.threshold > 0.f;
+  const bool early_exit = !NOISE && p.threshold > 0.f;
   for (;;) {
     int r = 0;
     if (lane == 0) r = atomicAdd(&a.w.counts->work, 1);
@@ -648,10 +699,13 @@ __global__ void __launch_bounds__(kAccWarps * kWarp, 5) k_lut_pixels(AccumArgs a
       continue;
     }
     float loss = 0.f;
-    RowStats rs{0.f, 0.f, false};
+    RowStats rs{0.f, 0.f, 0.f, false};
+    const auto nrm = [&] {
+      if constexpr (NOISE) return Draws(a.normals + (int64_t)r * (1 + 3 * H), H, lane);
+      else return NoDraws{};
+    }();
     if constexpr (!VJP) {
       // ---- front end on the output ticks (row + 1)
-      const float *nrm = a.normals ? a.normals + (int64_t)r * (1 + 3 * H) : nullptr;
       float *adc_dst = a.adc_out ? a.adc_out + (int64_t)r * H : nullptr;
       float *tick_dst = a.tick_out ? a.tick_out + (int64_t)r * H : nullptr;
       rs = warp_cumsum_charge(row + 1, T, p.t_sampling, lane);
@@ -661,7 +715,6 @@ __global__ void __launch_bounds__(kAccWarps * kWarp, 5) k_lut_pixels(AccumArgs a
       }
     }
     if constexpr (GRAD && !VJP) {
-      const float *nrm = a.normals ? a.normals + (int64_t)r * (1 + 3 * H) : nullptr;
       float *adc_dst = a.adc_out ? a.adc_out + (int64_t)r * H : nullptr;
       float *tick_dst = a.tick_out ? a.tick_out + (int64_t)r * H : nullptr;
       const bool swept =
@@ -682,7 +735,7 @@ __global__ void __launch_bounds__(kAccWarps * kWarp, 5) k_lut_pixels(AccumArgs a
       }
       loss = warp_sum(loss);
       __syncwarp();
-      fee_backward(p, row + 1, T, &sm.fee, sm.gint, swept, lane);
+      fee_backward(p, row + 1, T, rs, &sm.fee, sm.gint, swept, lane);
       if (lane == 0) row[0] = 0.f;
       __syncwarp();
     }
@@ -890,14 +943,14 @@ static size_t warp_smem_bytes(const LsimParams &) {
 }
 
 // Persistent grid: every SM filled to its occupancy limit.
-template <int MODE>
+template <int MODE, bool NOISE>
 static int grid_blocks(const LsimParams &p, int *blocks, size_t *smem_out) {
   const size_t smem = warp_smem_bytes<MODE>(p) * kAccWarps;
-  if (cudaFuncSetAttribute(k_lut_pixels<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+  if (cudaFuncSetAttribute(k_lut_pixels<MODE, NOISE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return LSIM_ERR_CUDA;
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lut_pixels<MODE>, kAccWarps * kWarp, smem) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lut_pixels<MODE, NOISE>, kAccWarps * kWarp, smem) !=
       cudaSuccess)
     return LSIM_ERR_CUDA;
   if (per_sm < 1) per_sm = 1;
@@ -908,21 +961,28 @@ static int grid_blocks(const LsimParams &p, int *blocks, size_t *smem_out) {
   return LSIM_OK;
 }
 
-template <int MODE>
-static int launch_mode(const AccumArgs &a0, cudaStream_t st) {
+template <int MODE, bool NOISE>
+static int launch_pixels(const AccumArgs &a0, cudaStream_t st) {
   int blocks = 0;
   size_t smem = 0;
-  int rc = grid_blocks<MODE>(a0.p, &blocks, &smem);
+  int rc = grid_blocks<MODE, NOISE>(a0.p, &blocks, &smem);
   if (rc != LSIM_OK) return rc;
   AccumArgs a = a0;
   a.warp_smem = (int)warp_smem_bytes<MODE>(a0.p);
   cudaEvent_t ev0, ev1;
   kernel_events(&ev0, &ev1);
   if (ev0 && cudaEventRecord(ev0, st) != cudaSuccess) return LSIM_ERR_CUDA;
-  k_lut_pixels<MODE><<<blocks, kAccWarps * kWarp, smem, st>>>(a);
+  k_lut_pixels<MODE, NOISE><<<blocks, kAccWarps * kWarp, smem, st>>>(a);
   if (cudaGetLastError() != cudaSuccess) return LSIM_ERR_CUDA;
   if (ev1 && cudaEventRecord(ev1, st) != cudaSuccess) return LSIM_ERR_CUDA;
   return LSIM_OK;
+}
+
+template <int MODE>
+static int launch_mode(const AccumArgs &a, cudaStream_t st) {
+  if constexpr (MODE != kModeWfs && MODE != kModeVjpWfs)
+    if (a.normals) return launch_pixels<MODE, true>(a, st);
+  return launch_pixels<MODE, false>(a, st);
 }
 
 int run_accum(AccumMode mode, const AccumArgs &a, cudaStream_t st) {

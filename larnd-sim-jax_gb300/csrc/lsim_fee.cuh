@@ -50,65 +50,102 @@ __device__ __forceinline__ float digitize_vjp(const LsimParams &p, float q, floa
   return ((g * gy) * (p.adc_counts / p.vref_minus_cm)) * gx * p.gain;
 }
 
-// Smallest and largest value of a lane's ticks (the largest with the next
-// lane's first tick), and whether the row suits the threshold path.
+// A row's cumulative charge is kept as its chunks' own prefix sums X (lane l:
+// ticks l per .. l per + per - 1) and each chunk's offset: C[i] = offset + X[i].
+// lo, hi: smallest and largest C of the lane's ticks (the largest with the
+// next lane's first tick); fast: whether the row suits the threshold path.
 struct RowStats {
-  float lo, hi;
+  float lo, hi, offset;
   bool fast;
 };
+__device__ __forceinline__ int chunk_ticks(int T) { return (T + kWarp - 1) / kWarp; }
+// i / per for i < 2048, the quotient's distance from an integer being at least 0.5 / per
+__device__ __forceinline__ int chunk_of(int i, int per) { return (int)(((float)i + 0.5f) * (1.0f / (float)per)); }
+// C[i], i possibly different in each lane (all lanes take part)
+__device__ __forceinline__ float row_charge(const float *X, const RowStats &rs, int T, int i) {
+  return __shfl_sync(0xffffffffu, rs.offset, chunk_of(i, chunk_ticks(T))) + X[i];
+}
 
 // Rows whose values stay below this (and are finite) take the threshold
 // path: no intermediate of the resets can overflow there.
 constexpr float kFeeFastMax = 1e30f;
 
-// In-place cumulative charge C[i] = sum_{j<=i} X[j]*ts over T ticks
-// (lane-contiguous chunks + warp exclusive scan of the chunk totals).
+// Cumulative charge C[i] = sum_{j<=i} X[j]*ts over T ticks: X becomes the
+// chunks' prefix sums, the offsets (a warp scan of the chunks' totals) and the
+// extremes of C are returned.  Adding an offset is monotone with its rounding,
+// so a chunk's extremes are the offset plus those of its prefix sums, and the
+// row is passed over once: a second pass that added the offsets took half of
+// this function's instructions, and the threshold path reads a few C only.
 __device__ __forceinline__ RowStats warp_cumsum_charge(float *X, int T, float ts, int lane) {
-  const int per = (T + kWarp - 1) / kWarp;
+  const int per = chunk_ticks(T);
   const int b = min(lane * per, T);
   const int e = min(b + per, T);
-  float s = 0.f;
+  float s = 0.f, lo = INFINITY, hi = -INFINITY;
   int i = b;
+#pragma unroll 1
   for (; i + 8 <= e; i += 8) {   // eight loads in flight ahead of the serial chain
     float x[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) x[q] = X[i + q];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) X[i + q] = s = fmaf(x[q], ts, s);
+    for (int q = 0; q < 8; ++q) {
+      X[i + q] = s = fmaf(x[q], ts, s);
+      lo = fminf(lo, s);
+      hi = fmaxf(hi, s);
+    }
   }
-  for (; i < e; ++i) X[i] = s = fmaf(X[i], ts, s);
+#pragma unroll 1
+  for (; i < e; ++i) {
+    X[i] = s = fmaf(X[i], ts, s);
+    lo = fminf(lo, s);
+    hi = fmaxf(hi, s);
+  }
   float incl = s;
+#pragma unroll 1
   for (int o = 1; o < kWarp; o <<= 1) {
     float y = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += y;
   }
-  const float offset = incl - s;
   RowStats st;
-  st.lo = INFINITY;
-  st.hi = -INFINITY;
-  float head = 0.f;              // the lane's first value
-  for (i = b; i < e; i += 8) {
-    float x[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) x[q] = i + q < e ? X[i + q] : 0.f;
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-      if (i + q < e) {
-        const float c = lane > 0 ? offset + x[q] : x[q];
-        X[i + q] = c;
-        if (i + q == b) head = c;
-        st.lo = fminf(st.lo, c);
-        st.hi = fmaxf(st.hi, c);
-      }
-  }
+  st.offset = lane > 0 ? incl - s : -0.f;     // -0 + x is x
+  st.lo = st.offset + lo;
+  st.hi = st.offset + hi;
   // a NaN in the row shows in its chunk's total or in the next chunks' offset
-  const bool ok = b >= e || (isfinite(s) && isfinite(offset) && st.lo > -kFeeFastMax && st.hi < kFeeFastMax);
-  const float nx = __shfl_down_sync(0xffffffffu, head, 1);
+  const bool ok = b >= e || (isfinite(s) && isfinite(st.offset) && st.lo > -kFeeFastMax && st.hi < kFeeFastMax);
+  const float nx = __shfl_down_sync(0xffffffffu, b < e ? st.offset + X[b] : 0.f, 1);
   if (lane < kWarp - 1 && e < T) st.hi = fmaxf(st.hi, nx);
   st.fast = __all_sync(0xffffffffu, ok);
   __syncwarp();
   return st;
 }
+
+// The cumulative charge itself, in place of the prefix sums.
+__device__ __forceinline__ void add_offsets(float *X, int T, const RowStats &rs, int lane) {
+  const int per = chunk_ticks(T), b = min(lane * per, T), e = min(b + per, T);
+  for (int i = b; i < e; ++i) X[i] = rs.offset + X[i];
+  __syncwarp();
+}
+
+// The noise draws of a row ([1 + 3H], or none), loaded once: lane l holds draws l and l + 32.
+struct Draws {
+  const float *src;
+  float a, b;
+  __device__ __forceinline__ Draws(const float *normals, int H, int lane) : src(normals), a(0.f), b(0.f) {
+    if (normals) {
+      if (lane < 1 + 3 * H) a = normals[lane];
+      if (lane + kWarp < 1 + 3 * H) b = normals[lane + kWarp];
+    }
+  }
+  __device__ __forceinline__ float operator[](int i) const {   // i the same in all lanes
+    return i < kWarp ? __shfl_sync(0xffffffffu, a, i) : __shfl_sync(0xffffffffu, b, i - kWarp);
+  }
+};
+static_assert(1 + 3 * LSIM_MAX_HITS <= 2 * kWarp, "two draws a lane");
+// ... and their absence, known when compiling
+struct NoDraws {
+  static constexpr const float *src = nullptr;
+  __device__ __forceinline__ float operator[](int) const { return 0.f; }
+};
 
 // C = cumsum(W * ts)  ->  dL/dW[i] = ts * sum_{j >= i} dL/dC[j], in place
 // (lane-contiguous chunks + warp suffix scan of the chunk totals).
@@ -117,16 +154,19 @@ __device__ __forceinline__ void warp_suffix_charge(float *G, int T, float ts, in
   const int b = lane * per;
   const int e = min(b + per, T);
   float s = 0.f;
+#pragma unroll 1
   for (int i = e - 1; i >= b; --i) {
     s += G[i];
     G[i] = s;
   }
   float incl = s;   // suffix sums across lanes
+#pragma unroll 1
   for (int o = 1; o < kWarp; o <<= 1) {
     float y = __shfl_down_sync(0xffffffffu, incl, o);
     if (lane + o < kWarp) incl += y;
   }
   const float offset = incl - s;
+#pragma unroll 1
   for (int i = b; i < e; ++i) G[i] = (offset + G[i]) * ts;
   __syncwarp();
 }
@@ -343,9 +383,11 @@ static __device__ __noinline__ void fee_backward_sweep(const LsimParams &p, floa
 // are replayed through the h resets.  Ticks, integrals and the adjoint are
 // bit for bit those of the sweep path, at a cost per hit of about 100
 // instructions per warp where a sweep of 2000 ticks takes about 1300.
-// simulate_stochastic on 30000 rows of 2000 ticks with noise: 809 -> 316 us;
-// the 64-event gradient step, where it is one phase of the pixel kernel:
-// 18.71 -> 17.92 ms.
+// simulate_stochastic on 30000 rows of 2000 ticks with noise, against the
+// sweeps: 809 -> 316 us; the 64-event gradient step, where it is one phase of
+// the pixel kernel: 18.71 -> 17.92 ms.
+// (The loops here are kept rolled: the code is hot inside the pixel kernels,
+// whose instructions do not fit in the cache.)
 
 // Total order of the floats as signed integers (and back).
 __device__ __forceinline__ int float_key(float x) {
@@ -358,6 +400,7 @@ __device__ __forceinline__ float key_float(int k) {
 
 // Charge of a tick after the first h resets (R in shared memory).
 __device__ __forceinline__ float replay_resets(float c, const float *R, int h) {
+#pragma unroll 1
   for (int k = 0; k < h; ++k) c = fmaxf(c - R[k], 0.f);
   return c;
 }
@@ -377,36 +420,49 @@ __device__ __forceinline__ Crossing crossing_thresholds(float guess, float base,
   const int key = lane == 0 ? kmin : (lane == kWarp - 1 ? kmax : k0 + lane - kWarp / 2);
   const float v = base + replay_resets(key_float(key), R, h);
   const unsigned m_from = __ballot_sync(0xffffffffu, v >= thr), m_above = __ballot_sync(0xffffffffu, v > thr);
-  auto resolve = [&](unsigned m, bool strict) {
-    if (m & 1u) return -kFeeFastMax;
-    if (!(m >> 31)) return (float)INFINITY;
-    int j = __ffs(m) - 1;                      // first lane that holds
-    int lo = __shfl_sync(0xffffffffu, key, j - 1), hi = __shfl_sync(0xffffffffu, key, j);
-    while ((uint32_t)hi - (uint32_t)lo > 1u) { // false at lo, true at hi; the span shrinks 33 times a round
-      const uint32_t span = (uint32_t)hi - (uint32_t)lo;
-      const uint32_t step = (uint32_t)(((uint64_t)span * (uint32_t)(lane + 1)) / (kWarp + 1));
-      const int kt = (int)((uint32_t)lo + (step > 0 ? step : 1u));
-      const float vt = base + replay_resets(key_float(kt), R, h);
-      const unsigned mt = __ballot_sync(0xffffffffu, strict ? vt > thr : vt >= thr);
-      j = mt ? __ffs(mt) - 1 : kWarp;
-      const int below = __shfl_sync(0xffffffffu, kt, j > 0 ? j - 1 : 0);
-      const int at = __shfl_sync(0xffffffffu, kt, j < kWarp ? j : 0);
-      if (j < kWarp) hi = at;
-      if (j > 0) lo = below;
+  Crossing x;
+#pragma unroll 1
+  for (int strict = 0; strict < 2; ++strict) {   // (rolled: the code is hot in a large kernel)
+    const unsigned m = strict ? m_above : m_from;
+    float found;
+    if (m & 1u) {
+      found = -kFeeFastMax;
+    } else if (!(m >> 31)) {
+      found = (float)INFINITY;
+    } else {
+      int j = __ffs(m) - 1;                      // first lane that holds
+      int lo = __shfl_sync(0xffffffffu, key, j - 1), hi = __shfl_sync(0xffffffffu, key, j);
+      while ((uint32_t)hi - (uint32_t)lo > 1u) { // false at lo, true at hi; the span shrinks 33 times a round
+        const uint32_t span = (uint32_t)hi - (uint32_t)lo;
+        const uint32_t step = (uint32_t)(((uint64_t)span * (uint32_t)(lane + 1)) / (kWarp + 1));
+        const int kt = (int)((uint32_t)lo + (step > 0 ? step : 1u));
+        const float vt = base + replay_resets(key_float(kt), R, h);
+        const unsigned mt = __ballot_sync(0xffffffffu, strict ? vt > thr : vt >= thr);
+        j = mt ? __ffs(mt) - 1 : kWarp;
+        const int below = __shfl_sync(0xffffffffu, kt, j > 0 ? j - 1 : 0);
+        const int at = __shfl_sync(0xffffffffu, kt, j < kWarp ? j : 0);
+        if (j < kWarp) hi = at;
+        if (j > 0) lo = below;
+      }
+      found = key_float(hi);
     }
-    return key_float(hi);
-  };
-  return Crossing{resolve(m_from, false), resolve(m_above, true)};
+    (strict ? x.above : x.from) = found;
+  }
+  return x;
 }
 
+// (C here and below: the chunks' prefix sums, RowStats.)
 // First i < T - 1 with C[i] < above and C[i + 1] >= from; T - 2 if none.
 __device__ __forceinline__ int warp_crossing(const float *C, int T, const RowStats &rs, const Crossing &x, int lane) {
-  const int per = (T + kWarp - 1) / kWarp;
+  const int per = chunk_ticks(T);
   for (unsigned m = __ballot_sync(0xffffffffu, rs.lo < x.above && rs.hi >= x.from); m; m &= m - 1) {
-    const int b = (__ffs(m) - 1) * per, n = min(per, T - 1 - b);
+    const int chunk = __ffs(m) - 1, b = chunk * per, n = min(per, T - 1 - b);
+    const float own = __shfl_sync(0xffffffffu, rs.offset, chunk);
+    const float next = __shfl_sync(0xffffffffu, rs.offset, (chunk + 1) & (kWarp - 1));
+#pragma unroll 1
     for (int j0 = 0; j0 < n; j0 += kWarp) {
       const int j = j0 + lane;
-      const bool hit = j < n && C[b + j] < x.above && C[b + j + 1] >= x.from;
+      const bool hit = j < n && own + C[b + j] < x.above && (j + 1 < per ? own : next) + C[b + j + 1] >= x.from;
       const unsigned bal = __ballot_sync(0xffffffffu, hit);
       if (bal) return b + j0 + __ffs(bal) - 1;
     }
@@ -417,13 +473,16 @@ __device__ __forceinline__ int warp_crossing(const float *C, int T, const RowSta
 // Forward self-trigger on C (left as it is); st: the hits' state (its R
 // serves every mode).  Outputs as fee_forward_sweep.  False (st and the
 // outputs hold nothing) when a noise draw is not finite.
+template <typename Noise>
 __device__ __forceinline__ bool fee_forward_threshold(const LsimParams &p, const float *C, int T, const RowStats &rs,
-                                                      const float *normals, float *adc_out, float *tick_out,
+                                                      const Noise &normals, float *adc_out, float *tick_out,
                                                       FeeState *st, float *raw_out, bool early_exit, int lane) {
   const float thr = p.threshold;
   const int H = p.max_adc_values;
-  float base = normals ? normals[0] * p.reset_noise : 0.f;
+  const bool noise = normals.src != nullptr;
+  float base = noise ? normals[0] * p.reset_noise : 0.f;
   float top = rs.hi;   // the row's largest value, and what the resets leave of it
+#pragma unroll 1
   for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
   float left = top, sum_r = 0.f;
   float my_raw = 0.f, my_tick = (float)(T - 2);   // lane h: hit h; the empty hit's values
@@ -435,14 +494,17 @@ __device__ __forceinline__ bool fee_forward_threshold(const LsimParams &p, const
     if (base + left >= thr)   // f_h is monotone: no tick reaches the threshold if the largest does not
       idx = warp_crossing(C, T, rs, crossing_thresholds((thr - base) + sum_r, base, thr, st->R, h, lane), lane);
     const int e = min(idx + 1 + p.fee_interval, T - 1), e2 = min(idx + 2 + p.fee_interval, T - 1);
-    const float c = replay_resets(C[lane & 1 ? e2 : e], st->R, h);
+    const float c = replay_resets(row_charge(C, rs, T, lane & 1 ? e2 : e), st->R, h);
     const float qvn = __shfl_sync(0xffffffffu, c, 0), R = __shfl_sync(0xffffffffu, c, 1);
     const float qv = base + qvn;
-    const float extra = normals ? normals[1 + 3 * h] * p.uncorr_noise : 0.f;
+    const float extra = noise ? normals[1 + 3 * h] * p.uncorr_noise : 0.f;
     float adc = (qvn != 0.f) ? (qv + extra) : qvn;
     const bool cond = (adc < thr) || (idx == T - 2);
     if (cond) adc = 0.f;
-    if (normals) base = cond ? normals[3 + 3 * h] * p.uncorr_noise : normals[2 + 3 * h] * p.reset_noise;
+    if (noise) {
+      const float d2 = normals[2 + 3 * h], d3 = normals[3 + 3 * h];
+      base = cond ? d3 * p.uncorr_noise : d2 * p.reset_noise;
+    }
     if (lane == h) {
       my_raw = adc;
       my_tick = cond ? (float)(T - 2) : (float)idx;
@@ -482,8 +544,8 @@ __device__ __forceinline__ bool fee_forward_threshold(const LsimParams &p, const
 // its replayed charge does, so going back over a reset only drops values;
 // their sum is formed in the order of the sweeps (per owner of a tick's
 // 4-tick group in ascending order, then across the warp).
-__device__ __forceinline__ void fee_backward_threshold(const LsimParams &p, float *C, int T, const FeeState *st,
-                                                       const float *gint, int lane) {
+__device__ __forceinline__ void fee_backward_threshold(const LsimParams &p, float *C, int T, const RowStats &rs,
+                                                       const FeeState *st, const float *gint, int lane) {
   static_assert(2 * LSIM_MAX_HITS <= kWarp, "two entries per hit");
   const int n_done = st->n_done, mine = lane >> 1;
   const bool used = mine < n_done;
@@ -491,16 +553,15 @@ __device__ __forceinline__ void fee_backward_threshold(const LsimParams &p, floa
   const unsigned same = __match_any_sync(0xffffffffu, tick);   // every lane takes part
   const bool holds = used && lane == __ffs(same) - 1;
   uint32_t keep = 0u;      // bit h: the tick survives reset h
-  float c = used ? C[tick] : 0.f;
+  float c = row_charge(C, rs, T, used ? tick : 0);
+#pragma unroll 1
   for (int h = 0; h < n_done; ++h) {
     const float d = c - st->R[h];
     keep |= d < 0.f ? 0u : 1u << h;
     c = fmaxf(d, 0.f);
   }
-  __syncwarp();
-  float4 *C4 = reinterpret_cast<float4 *>(C);
-  for (int i = 4 * lane; i < T; i += kFeePass) C4[i / 4] = make_float4(0.f, 0.f, 0.f, 0.f);
   float g = 0.f;
+#pragma unroll 1
   for (int h = n_done - 1; h >= 0; --h) {
     if (!((keep >> h) & 1u)) g = 0.f;
     float S = 0.f;
@@ -518,6 +579,10 @@ __device__ __forceinline__ void fee_backward_threshold(const LsimParams &p, floa
     if (holds && tick == t0 && !st->cond[h]) g += gint[h];
   }
   __syncwarp();
+  float4 *C4 = reinterpret_cast<float4 *>(C);
+#pragma unroll 1
+  for (int i = 4 * lane; i < T; i += kFeePass) C4[i / 4] = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncwarp();
   if (holds) C[tick] = g;
   __syncwarp();
   warp_suffix_charge(C, T, p.t_sampling, lane);
@@ -527,22 +592,25 @@ __device__ __forceinline__ void fee_backward_threshold(const LsimParams &p, floa
 // applies, else the sweeps (which use the row up).  `masks`: whether the
 // sweeps record their reset masks for the adjoint.  Returns whether the row
 // was swept, which fee_backward needs to know.
+template <typename Noise>
 __device__ __forceinline__ bool fee_forward(const LsimParams &p, float *C, int T, const RowStats &rs,
-                                            const float *normals, float *adc_out, float *tick_out, FeeState *st,
+                                            const Noise &normals, float *adc_out, float *tick_out, FeeState *st,
                                             bool masks, float *raw_out, bool early_exit, int lane) {
   if (rs.fast && fabsf(p.threshold) < kFeeFastMax &&
       fee_forward_threshold(p, C, T, rs, normals, adc_out, tick_out, st, raw_out, early_exit, lane))
     return false;
-  fee_forward_sweep(p, C, T, normals, adc_out, tick_out, masks ? st : nullptr, raw_out, early_exit, lane);
+  add_offsets(C, T, rs, lane);
+  fee_forward_sweep(p, C, T, normals.src, adc_out, tick_out, masks ? st : nullptr, raw_out, early_exit, lane);
   return true;
 }
 
-__device__ __forceinline__ void fee_backward(const LsimParams &p, float *C, int T, const FeeState *st,
+__device__ __forceinline__ void fee_backward(const LsimParams &p, float *C, int T, const RowStats &rs,
+                                             const FeeState *st,
                                              const float *gint, bool swept, int lane) {
   if (swept)
     fee_backward_sweep(p, C, T, st, gint, lane);
   else
-    fee_backward_threshold(p, C, T, st, gint, lane);
+    fee_backward_threshold(p, C, T, rs, st, gint, lane);
 }
 
 }  // namespace lsim
