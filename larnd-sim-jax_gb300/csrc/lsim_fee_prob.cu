@@ -38,12 +38,14 @@ constexpr float kProbFloor = -1000.0f;
 // jax.scipy.special.ndtr / log_ndtr in float32 (the published piecewise
 // form: erf near zero and erfc in the tails for ndtr; -ndtr(-x) above 5,
 // log(ndtr(x)) down to -10, the order-3 asymptotic series below).
-// ndtr, log_ndtr and log_diff_ndtr's log term are called, not inlined:
-// inlined at every call site of the per-path loops their erf/erfc/log
-// bodies overflowed the instruction cache (the beam search ran 2.0x and
-// its adjoint 2.2x slower, with identical results).
+// log_ndtr below 15 is called, not inlined: inlined at every call site of the
+// per-path loops its erf/erfc/log body overflowed the instruction cache (the
+// beam search ran 2.0x and its adjoint 2.2x slower, with identical results).
+// What surrounds it is inlined: the largest arguments, which need nothing, do
+// not pay for a call.  Lanes differ in their branches, so both signs share one
+// ndtr and both directions of a log-sum-exp one exp.
 
-__device__ __noinline__ float ndtr_f(float x) {
+__device__ __forceinline__ float ndtr_f(float x) {
   const float hs2 = 0.70710678118654752f;
   const float w = x * hs2;
   const float z = fabsf(w);
@@ -51,11 +53,11 @@ __device__ __noinline__ float ndtr_f(float x) {
   return 0.5f * y;
 }
 
-__device__ __noinline__ float log_ndtr_f(float x) {
-  // above 15, erfc(x / sqrt 2) < 1e-50 is 0 in float32: -ndtr(-x) = -0
-  if (x > 15.0f) return -0.0f;
-  if (x > 5.0f) return -ndtr_f(-x);
-  if (x > -10.0f) return logf(ndtr_f(x));
+__device__ __noinline__ float log_ndtr_below_15(float x) {
+  if (x > -10.0f) {
+    const float n = ndtr_f(x > 5.0f ? -x : x);
+    return x > 5.0f ? -n : logf(n);
+  }
   const float x2 = x * x;
   const float log_scale = (-(x2 / 2.0f) - logf(-x)) - 0.918938533204672742f;   // 0.5 log(2 pi)
   const float x4 = x2 * x2;
@@ -64,6 +66,9 @@ __device__ __noinline__ float log_ndtr_f(float x) {
   const float even = 3.0f / x4;
   return log_scale + logf((1.0f + even) - odd);
 }
+
+// above 15, erfc(x / sqrt 2) < 1e-50 is 0 in float32: -ndtr(-x) = -0
+__device__ __forceinline__ float log_ndtr_f(float x) { return x > 15.0f ? -0.0f : log_ndtr_below_15(x); }
 
 // jax.nn.softplus = logaddexp(y, 0) = max(y, 0) + log1p(exp(-|y|)).  For
 // |y| > 110 exp(-|y|) is 0 in float32, so the value is exactly max(y, 0).
@@ -75,7 +80,7 @@ __device__ __forceinline__ float softplus_f(float y) {
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
 
 // The clamped log(1 - exp(safe)) term of log_diff_ndtr.
-__device__ __noinline__ float ldn_log_term(float safe) {
+__device__ __forceinline__ float ldn_log_term(float safe) {
   const float neg = -expm1f(safe);
   const float neg_safe = 1e-30f + softplus_f((neg - 1e-30f) * 1e10f) / 1e10f;
   // neg_safe >= 1e-30, so lt >= -69.1 and the clamp's softplus argument
@@ -92,18 +97,21 @@ __device__ __forceinline__ float log_diff_ndtr_f(float a, float b, float la, flo
   if (a == b) return 0.5f * (la + term_m1) + 0.5f * kProbFloor;
   const float lts = a > b ? ldn_log_term(lb - la) : term_m1;
   const float lp = la + lts;
+  if ((a - b) * 1000.0f > 20.0f) return lp;     // the gate is 1 in float32 (1 + e^-20)
   const float w = sigmoid_f((a - b) * 1000.0f);
   return w * lp + (1.0f - w) * kProbFloor;
 }
 
 // online log-sum-exp: m = running maximum, s = sum of exp(x - m)
-// (exp of arguments below -110 is 0 in float32 and is skipped)
+// (exp of arguments below -110 is 0 in float32)
 __device__ __forceinline__ void lse_add(float &m, float &s, float x) {
-  if (x > m) {
-    s = m - x > -110.0f ? s * expf(m - x) + 1.0f : 1.0f;
+  const float d = x - m;
+  const float e = fabsf(d) < 110.0f ? expf(-fabsf(d)) : 0.0f;   // one for both directions: lanes differ
+  if (d > 0.0f) {
+    s = s * e + 1.0f;
     m = x;
-  } else if (x - m > -110.0f) {
-    s += expf(x - m);
+  } else {
+    s += e;
   }
 }
 
@@ -252,7 +260,7 @@ constexpr float kWeakRise = 1.4f, kWeakMost = -190.0f;
 //   whose dist term is above kProbFar;
 // * a pixel whose paths have all become improbable beyond kProbDead stops.
 // Bound by instruction issue in the special functions.  Values and gradient of
-// 1500 dense rows: 42.4 -> 6.5 ms (10.1 before the adjoint below); distributions of 1000 rows: 8.8 -> 5.2 ms.
+// 1500 dense rows: 42.4 -> 6.1 ms (10.1 before the adjoint below); distributions of 1000 rows: 8.8 -> 5.0 ms.
 template <bool kDist>
 __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob(ProbArgs a) {
   extern __shared__ __align__(16) float sm[];
