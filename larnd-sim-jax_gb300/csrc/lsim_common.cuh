@@ -19,7 +19,6 @@ constexpr int kMainSub = 5;              // main-bin LUT sub-positions (nb_bins_
 constexpr int kMaxSlotSegments = (1 << 23) - 1;   // segments sharing one principal pixel
 constexpr int kWinSamples = 160;         // padded window samples k = -1 .. 158 (signal_length <= 158)
 constexpr int kScanTile = 2048;          // slots per scan block
-constexpr int kSortLocal = 64;           // slot lists up to this length are sorted by one thread
 constexpr int kThetaDerived = 16;
 constexpr int kScanThreads = 256;
 
@@ -135,7 +134,6 @@ struct Workspace {
   int32_t *key, *pid;
   int32_t *cnt, *off, *cursor;
   int32_t *seg_list, *pix_slot, *em1_slot;
-  int32_t *big_slots;       // slots with more than kSortLocal segments (sorted by a block each)
   float *theta_derived;     // fit parameters and derived quantities for lsim_lut_stage1_theta (kThetaDerived)
   int32_t *heavy;           // pixels with many contributions, handed out first (count in counts->reserved[0])
   uint8_t *heavy_flag;      // per valid pixel: 1 if it is in the heavy list
@@ -181,7 +179,6 @@ inline Workspace carve_workspace(void *base, const LsimParams &p, int64_t n_rows
   size_t o_list = take(4 * (size_t)n_rows);
   size_t o_pixs = take(4 * (size_t)n_rows);
   size_t o_em1 = take(4 * (size_t)n_rows);
-  size_t o_big = take(4 * ((size_t)n_rows / (kSortLocal + 1) + 1));
   size_t o_theta = take(4 * (size_t)kThetaDerived);
   size_t o_heavy = take(4 * (size_t)n_rows);
   size_t o_hflag = take((size_t)n_rows);
@@ -212,7 +209,6 @@ inline Workspace carve_workspace(void *base, const LsimParams &p, int64_t n_rows
   w.seg_list = (int32_t *)(b + o_list);
   w.pix_slot = (int32_t *)(b + o_pixs);
   w.em1_slot = (int32_t *)(b + o_em1);
-  w.big_slots = (int32_t *)(b + o_big);
   w.theta_derived = (float *)(b + o_theta);
   w.heavy = (int32_t *)(b + o_heavy);
   w.heavy_flag = (uint8_t *)(b + o_hflag);

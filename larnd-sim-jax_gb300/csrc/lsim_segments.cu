@@ -510,118 +510,50 @@ __global__ void k_scan_final(const int32_t *__restrict__ cnt, int64_t G, Grid g,
   }
 }
 
-// Scatter segment indices into their slot ranges.
+// Scatter segment indices into their slot ranges, in any order.
 __global__ void k_scatter(const int32_t *__restrict__ key, int64_t n_rows, const int32_t *__restrict__ off,
-                          int32_t *__restrict__ cursor, int32_t *__restrict__ seg_list) {
+                          int32_t *__restrict__ cursor, int32_t *__restrict__ list) {
   int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s >= n_rows) return;
   int32_t k = key[s];
   if (k < 0) return;
   int pos = off[k] + atomicAdd(&cursor[k], 1);
-  seg_list[pos] = (int32_t)s;
+  list[pos] = (int32_t)s;
 }
 
-// Sort each slot's segment list ascending so accumulation order, and hence
-// every float32 result, is deterministic.  Lists of up to kSortLocal
-// segments are sorted here by one thread; longer ones are queued for
-// k_sort_big_slots.
-// List-ordered copies of the compact neighbour-pass records (LUT mode;
-// lnb null in parametrised mode): entry i of the slot lists gets the record
-// of segment seg_list[i].
-__device__ __forceinline__ void copy_list_records(const Workspace &w, int64_t pos, int32_t s) {
-  if (!w.lnb) return;
-  w.lnb[pos] = w.segn[s];
-  w.lna[pos] = w.segna[s];
-}
-
-__global__ void k_sort_slots(const int32_t *__restrict__ cnt, const int32_t *__restrict__ off, int64_t G,
-                             int32_t *__restrict__ seg_list, int32_t *__restrict__ big_slots, LsimCounts *counts,
+// Each slot's segment list in ascending order, so accumulation order, and
+// hence every float32 result, is deterministic.  A thread per segment counts
+// the segments before it in its slot's unordered list (neighbouring segments
+// share slots, so the reads are mostly broadcasts) and writes its own entry,
+// and in LUT mode (lnb not null) its compact neighbour-pass records there.
+// Latency-bound: a thread per slot that sorted its list left most threads
+// without a slot and walked long lists alone, with a second kernel for the
+// longest (64 events 186, one event 19 us; 46 and 5 us so).
+__global__ void k_rank_slots(const int32_t *__restrict__ key, int64_t n_rows, const int32_t *__restrict__ cnt,
+                             const int32_t *__restrict__ off, const int32_t *__restrict__ list, LsimCounts *counts,
                              Workspace w) {
-  int64_t slot = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int c = slot < G ? cnt[slot] : 0;
+  const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int32_t k = s < n_rows ? key[s] : -1;
+  const int c = k >= 0 ? cnt[k] : 0;
   // one atomic per warp for the largest slot (a shared counter is hot)
   const int cmax = __reduce_max_sync(0xffffffffu, c);
   if ((threadIdx.x % kWarp) == 0 && cmax > 1) {
-    atomicMax(&counts->max_slot, cmax);
+    if (cmax > *(volatile int32_t *)&counts->max_slot) atomicMax(&counts->max_slot, cmax);
     if (cmax > kMaxSlotSegments) atomicCAS(&counts->status, 0, (int)LSIM_ERR_CAPACITY);
   }
   if (c <= 0) return;
-  const int64_t o = off[slot];
-  int32_t *l = seg_list + o;
-  if (c == 1) {
-    copy_list_records(w, o, l[0]);
-    return;
+  const int64_t o = off[k];
+  int rank = 0;
+  if (c > kMaxSlotSegments) {        // refused by the status: any order
+    rank = atomicSub(&w.cursor[k], 1) - 1;
+  } else {
+#pragma unroll 8
+    for (int i = 0; i < c; ++i) rank += __ldg(list + o + i) < (int32_t)s;
   }
-  if (c > kSortLocal) {
-    big_slots[atomicAdd(&counts->n_big_slots, 1)] = (int32_t)slot;
-    return;
-  }
-  {
-    // short lists (nearly all): insertion sort in a thread-local copy
-    int32_t v[kSortLocal];
-    for (int i = 0; i < c; ++i) v[i] = l[i];
-    for (int i = 1; i < c; ++i) {
-      const int32_t x = v[i];
-      int j = i - 1;
-      while (j >= 0 && v[j] > x) { v[j + 1] = v[j]; --j; }
-      v[j + 1] = x;
-    }
-    for (int i = 0; i < c; ++i) {
-      l[i] = v[i];
-      copy_list_records(w, o + i, v[i]);
-    }
-  }
-}
-
-// One block per queued long list: bitonic sort in shared memory for lists
-// up to kSortBig entries, a block-wide odd-even transposition sort in place
-// beyond (lists that long do not occur in practice).
-constexpr int kSortBig = 8192;
-constexpr int kSortThreads = 256;
-
-__global__ void __launch_bounds__(kSortThreads) k_sort_big_slots(const int32_t *__restrict__ cnt,
-                                                                 const int32_t *__restrict__ off,
-                                                                 int32_t *__restrict__ seg_list,
-                                                                 const int32_t *__restrict__ big_slots,
-                                                                 const LsimCounts *counts, Workspace w) {
-  __shared__ int32_t sh[kSortBig];
-  const int nbig = counts->n_big_slots;
-  for (int b = blockIdx.x; b < nbig; b += gridDim.x) {
-    const int64_t slot = big_slots[b];
-    const int c = cnt[slot];
-    int32_t *l = seg_list + off[slot];
-    if (c <= kSortBig) {
-      int n2 = 1;
-      while (n2 < c) n2 <<= 1;
-      for (int i = threadIdx.x; i < n2; i += kSortThreads) sh[i] = i < c ? l[i] : INT32_MAX;
-      __syncthreads();
-      for (int k = 2; k <= n2; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-          for (int i = threadIdx.x; i < n2; i += kSortThreads) {
-            const int ij = i ^ j;
-            if (ij > i) {
-              const bool up = (i & k) == 0;
-              const int32_t a = sh[i], d = sh[ij];
-              if ((a > d) == up) { sh[i] = d; sh[ij] = a; }
-            }
-          }
-          __syncthreads();
-        }
-      for (int i = threadIdx.x; i < c; i += kSortThreads) {
-        l[i] = sh[i];
-        copy_list_records(w, off[slot] + i, sh[i]);
-      }
-    } else {
-      for (int phase = 0; phase < c; ++phase) {
-        for (int i = 2 * threadIdx.x + (phase & 1); i + 1 < c; i += 2 * kSortThreads) {
-          const int32_t a = l[i], d = l[i + 1];
-          if (a > d) { l[i] = d; l[i + 1] = a; }
-        }
-        __syncthreads();
-      }
-      for (int i = threadIdx.x; i < c; i += kSortThreads) copy_list_records(w, off[slot] + i, l[i]);
-    }
-    __syncthreads();
+  w.seg_list[o + rank] = (int32_t)s;
+  if (w.lnb) {
+    w.lnb[o + rank] = w.segn[s];
+    w.lna[o + rank] = w.segna[s];
   }
 }
 
@@ -662,12 +594,11 @@ int run_pixel_map(const LsimParams &p, const Workspace &w0, const Grid &g, int64
     k_scan_final<<<(unsigned)nscan, kScanThreads, 0, st>>>(w.cnt, g.G, g, w.scan_blocks, w.off, w.pix_slot,
                                                           w.em1_slot);
   }
-  if (n_rows > 0) k_scatter<<<(unsigned)((n_rows + 255) / 256), 256, 0, st>>>(w.key, n_rows, w.off, w.cursor, w.seg_list);
-  if (g.G > 0) {
-    k_sort_slots<<<(unsigned)((g.G + 255) / 256), 256, 0, st>>>(w.cnt, w.off, g.G, w.seg_list, w.big_slots,
-                                                                 w.counts, w);
-    k_sort_big_slots<<<(unsigned)(device_sm_count() * 4), kSortThreads, 0, st>>>(w.cnt, w.off, w.seg_list,
-                                                                                w.big_slots, w.counts, w);
+  if (n_rows > 0) {
+    int32_t *unordered = w.seg_order;   // written again by the passes that use it
+    const unsigned nb = (unsigned)((n_rows + 255) / 256);
+    k_scatter<<<nb, 256, 0, st>>>(w.key, n_rows, w.off, w.cursor, unordered);
+    k_rank_slots<<<nb, 256, 0, st>>>(w.key, n_rows, w.cnt, w.off, unordered, w.counts, w);
   }
   return LSIM_OK;
 }
