@@ -46,9 +46,9 @@ N_NEIGH, SIG_LEN = 4, 150
 PERTURB_SEED = 1234
 L2_FLUSH_BYTES = 512 << 20
 CPU_CHUNK = 150          # segments per CPU reference sample (one run per process)
-KERNELS_PER_STEP = 20   # stage 1: reset, segments, 3 scan, scatter, 2 sort; gradient: 3 template-order kernels,
-                        # main records, heavy-pixel list, target index, pixels, main adjoint, 2 record reductions,
-                        # target-only, finalize (counted in the launch list of the step)
+KERNELS_PER_STEP = 16   # stage 1: reset, segments, 3 scan, scatter, rank; gradient: pass reset and preparation,
+                        # 2 template-order kernels, main records, pixels, main adjoint, partial sums, finalize
+                        # (counted in the launch list of the step)
 # DRAM bytes per simulated pixel of one k_lut_pixels<grad> launch, from an
 # ncu capture of the 8-event case of this workload (22,066 pixels; traffic
 # scales with the pixel count)
@@ -1171,9 +1171,9 @@ def run_loss(args):
                       "same_event_pair_terms": pairs, "l2": "working set < L2 (hits only)"},
            "e2e": {"value": n / e2e_s, "unit": "hits/s", "ms_per_step": e2e_s * 1e3,
                    "h2d_bytes_per_step": int(sum(a.numel() * 4 for a in host)), "d2h_bytes_per_step": 4 + 8 * n},
-           "roofline": {"bound": "issue", "kernel": "k_rbf_rows",
-                        "note": "pairwise exp per same-event pair; inputs are a few MB"},
-           "gpu_launches": 7 * args.steps, "clocks": clk}
+           "roofline": {"bound": "issue", "kernel": "k_pair_rows",
+                        "note": "pairwise exp per pair of nearby hits; inputs are a few MB"},
+           "gpu_launches": 5 * args.steps, "clocks": clk}
     if not args.no_cpu_baseline:
         from oracle import losses_np as L
         e0 = (ev == 0).cpu().numpy()
