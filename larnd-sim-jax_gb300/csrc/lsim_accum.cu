@@ -735,7 +735,7 @@ __global__ void __launch_bounds__(kAccWarps * kWarp, 5) k_lut_pixels(AccumArgs a
       }
       loss = warp_sum(loss);
       __syncwarp();
-      fee_backward(p, row + 1, T, rs, &sm.fee, sm.gint, swept, lane);
+      fee_backward<1>(p, row + 1, T, rs, &sm.fee, sm.gint, swept, lane);
       if (lane == 0) row[0] = 0.f;
       __syncwarp();
     }

@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(kFeeWarps * kWarp, 6)
     __syncwarp();
     if (lane < H) gint[wid][lane] = digitize_vjp(p, st.raw[lane], g_adc[r * H + lane]);
     __syncwarp();
-    fee_backward(p, C, T, rs, &st, gint[wid], swept, lane);
+    fee_backward<8>(p, C, T, rs, &st, gint[wid], swept, lane);
     const float4 *c4 = reinterpret_cast<const float4 *>(C);
     float4 *d4 = reinterpret_cast<float4 *>(g_wfs + r * (int64_t)T);
     for (int i = lane; i < T / 4; i += kWarp) d4[i] = c4[i];

@@ -149,12 +149,15 @@ struct NoDraws {
 
 // C = cumsum(W * ts)  ->  dL/dW[i] = ts * sum_{j >= i} dL/dC[j], in place
 // (lane-contiguous chunks + warp suffix scan of the chunk totals).
+// kUnroll: 1 in the pixel kernels, whose instructions do not fit in the cache;
+// k_fee_vjp takes 8 (244 against 212 us for 16 events' rows of 2000 ticks).
+template <int kUnroll>
 __device__ __forceinline__ void warp_suffix_charge(float *G, int T, float ts, int lane) {
-  const int per = (T + kWarp - 1) / kWarp;
+  const int per = chunk_ticks(T);
   const int b = lane * per;
   const int e = min(b + per, T);
   float s = 0.f;
-#pragma unroll 1
+#pragma unroll kUnroll
   for (int i = e - 1; i >= b; --i) {
     s += G[i];
     G[i] = s;
@@ -166,7 +169,7 @@ __device__ __forceinline__ void warp_suffix_charge(float *G, int T, float ts, in
     if (lane + o < kWarp) incl += y;
   }
   const float offset = incl - s;
-#pragma unroll 1
+#pragma unroll kUnroll
   for (int i = b; i < e; ++i) G[i] = (offset + G[i]) * ts;
   __syncwarp();
 }
@@ -368,7 +371,7 @@ static __device__ __noinline__ void fee_backward_sweep(const LsimParams &p, floa
     }
     __syncwarp();
   }
-  warp_suffix_charge(G, T, p.t_sampling, lane);
+  warp_suffix_charge<1>(G, T, p.t_sampling, lane);
 }
 
 // ---------------------------------------------------------------- threshold path
@@ -544,6 +547,7 @@ __device__ __forceinline__ bool fee_forward_threshold(const LsimParams &p, const
 // its replayed charge does, so going back over a reset only drops values;
 // their sum is formed in the order of the sweeps (per owner of a tick's
 // 4-tick group in ascending order, then across the warp).
+template <int kUnroll>
 __device__ __forceinline__ void fee_backward_threshold(const LsimParams &p, float *C, int T, const RowStats &rs,
                                                        const FeeState *st, const float *gint, int lane) {
   static_assert(2 * LSIM_MAX_HITS <= kWarp, "two entries per hit");
@@ -585,7 +589,7 @@ __device__ __forceinline__ void fee_backward_threshold(const LsimParams &p, floa
   __syncwarp();
   if (holds) C[tick] = g;
   __syncwarp();
-  warp_suffix_charge(C, T, p.t_sampling, lane);
+  warp_suffix_charge<kUnroll>(C, T, p.t_sampling, lane);
 }
 
 // The front end on a row of cumulative charge: the threshold path where it
@@ -604,13 +608,14 @@ __device__ __forceinline__ bool fee_forward(const LsimParams &p, float *C, int T
   return true;
 }
 
+template <int kUnroll>
 __device__ __forceinline__ void fee_backward(const LsimParams &p, float *C, int T, const RowStats &rs,
                                              const FeeState *st,
                                              const float *gint, bool swept, int lane) {
   if (swept)
     fee_backward_sweep(p, C, T, st, gint, lane);
   else
-    fee_backward_threshold(p, C, T, rs, st, gint, lane);
+    fee_backward_threshold<kUnroll>(p, C, T, rs, st, gint, lane);
 }
 
 }  // namespace lsim

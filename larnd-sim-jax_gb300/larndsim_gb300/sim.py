@@ -507,9 +507,9 @@ class _FeeFn(torch.autograd.Function):
         (w,) = ctx.saved_tensors
         lib = _abi.load()
         P, T = w.shape
-        g = torch.zeros_like(w)
         if g_adc is None:
-            return g, None, None
+            return torch.zeros_like(w), None, None
+        g = torch.empty_like(w)      # every row is written
         ga = g_adc.to(torch.float32).contiguous()
         ws = torch.empty(lib.lsim_fee_vjp_workspace_bytes(P), dtype=torch.uint8, device=w.device)
         _abi.check(lib, lib.lsim_fee_vjp(ctx.lp, _ptr(w), P, T, _ptr(ctx.normals), _ptr(ga), _ptr(g), _ptr(ws),
