@@ -12,6 +12,8 @@
 // least 1e5 - (detector size) apart in x, so their kernel value
 // exp(-d / (2 sigma^2)) is exactly 0 in float32: inputs ordered by event (as
 // the hit compaction emits them) make the cost per-event quadratic.
+#include <cmath>
+
 #include "lsim_internal.cuh"
 
 namespace lsim {
@@ -61,18 +63,21 @@ __global__ void k_chunk_events(const int32_t *__restrict__ event, int64_t n, int
 // Split: one warp owns a tile of 64 row hits (two per lane, advanced
 // together in packed f32x2 operations) and walks the columns in chunks of
 // 32, each staged once per warp in shared memory with its values doubled up
-// for the packed operands.  Hits come in pixel order, so a chunk is short
-// in y and x: chunks whose bounding box lies so far from the tile's that
-// every K_ij is below 2^-kCutMse (mse_adc, 9.4 sigma) or 2^-kCutNll (nll,
-// 11.8 sigma) are passed over.  What that leaves out of an mse_adc sum is
-// below N w 2^-64, next to a_i >= w_i; nll divides by lambda + 1e-10, so its
-// line lies where N 2^-100 stays below 1e-10 2^-24 for any N < 2^40.  About
-// half of the chunks of the 64-event batch remain at 9.4 sigma (a spatial
-// sort of the hits does not lower that: 32 hits fill a box of some cm).
-// Chunks with no event in common are passed over as before (their K is
-// exactly 0), found 32 at a time by the lanes over a two-level list of
-// event ranges.  A chunk or tile that holds an infinity or a NaN has an
-// infinite box and is never passed over.
+// for the packed operands.  Chunks with no event in common are passed over
+// (their K is exactly 0), found 32 at a time by the lanes over a two-level
+// list of event ranges.  Hits come in pixel order, so a chunk is short in y
+// and x: chunks whose bounding box lies so far from the tile's that every
+// K_ij is below 2^-kCutMse (mse_adc, 9.4 sigma) or 2^-kCutNll (nll, 11.8
+// sigma) are passed over as well, about half of them on the 64-event batch
+// (a spatial sort of the hits does not lower that: 32 hits fill a box of some
+// cm).  A chunk or tile that holds an infinity or a NaN has an infinite box
+// and is never passed over.
+//
+// What is left out so is bounded as the tile goes along (weights of a chunk
+// times the largest K its box allows; kernel values below 2^-126, which the
+// exponential flushes, the same way).  Where a row's sums are not 2^26 times
+// that bound - a hit far from all others - they are formed again with expf,
+// over every chunk whose K is not 0 in float32.
 //
 // A row's sums are formed per 32 chunks and those added up: at 64 events the
 // z gradient's error against float64 is 1.9e-7 of its size (8.4e-7 with one
@@ -81,7 +86,7 @@ __global__ void k_chunk_events(const int32_t *__restrict__ event, int64_t n, int
 // Bound by float32 issue: 10 packed operations and 2 exponentials per
 // column for two rows, against about 23 operations per pair before.
 // mse_adc with its gradient on the hits of 64 events (0.7M x 0.7M): 34.9 ->
-// 5.91 ms; nll_loss on those of 8 events: 1.78 -> 0.42 ms.
+// 5.87 ms; nll_loss on those of 8 events: 1.78 -> 0.43 ms.
 // Few rows leave the chip idle, so the columns are dealt to pair_slices()
 // warps per tile, whose partial sums are added in slice order.
 constexpr int kPairTile = 64;     // row hits per warp
@@ -91,15 +96,19 @@ constexpr int kPairWarps = 4;     // warps per block
 constexpr int kPairMaxSlices = 16;
 constexpr int kPairWantWarps = 4864;   // 152 SMs x 32 warps: below this the columns are sliced
 constexpr float kCutMse = 64.f, kCutNll = 100.f;
+constexpr float kCutZero = 150.f;      // 2^-150 and below round to 0
+constexpr float kLeftOut = 67108864.f; // 2^26: a quarter of a float32's last place
+constexpr float kTiny = 1.1754944e-38f; // 2^-126, the smallest kernel value the fast exponential forms
 
 // One set of hits as the pair kernel reads it: stacked coordinates and
 // weight per hit (rounded up to whole chunks, weight 0 past the end), per
-// chunk the event range and the box, per 32 chunks the event range.
+// chunk the event range, the box and the sum of |w|, per 32 chunks the event range.
 struct PairSet {
   float4 *h;          // (stacked x, y, z, w)
   float *q;           // 4th coordinate or null
   int2 *ev, *ev_up;
   float4 *lo, *hi;    // box of a chunk (x, y, z, q)
+  float *wsum;
   int64_t n;
 };
 
@@ -129,11 +138,20 @@ __device__ __forceinline__ float warp_max(float v) {
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
 
-// Fills both sets: blocks [0, blocks_a) of 32 chunks belong to a, the rest to b.
+// Fills both sets: blocks [0, blocks_a) of 32 chunks belong to a, the rest to
+// b; clears the tiles' counters.
 __global__ void __launch_bounds__(kPairSuper * kPairChunk) k_pair_prepare(PairSource sa, PairSet a, int64_t blocks_a,
-                                                                          PairSource sb, PairSet b) {
+                                                                          PairSource sb, PairSet b, int32_t *done,
+                                                                          int64_t n_done) {
   __shared__ int2 ranges[kPairSuper];
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_done; i += (int64_t)gridDim.x * blockDim.x)
+    done[i] = 0;
   const bool first = blockIdx.x < blocks_a;
   const PairSource &src = first ? sa : sb;
   const PairSet &set = first ? a : b;
@@ -153,6 +171,7 @@ __global__ void __launch_bounds__(kPairSuper * kPairChunk) k_pair_prepare(PairSo
   }
   const bool odd = ok && !(isfinite(x) && isfinite(y) && isfinite(z) && isfinite(q) && isfinite(w));
   const bool any_odd = __any_sync(0xffffffffu, odd);
+  const float wsum = warp_sum(fabsf(w));
   elo = __reduce_min_sync(0xffffffffu, elo);
   ehi = __reduce_max_sync(0xffffffffu, ehi);
   const float inf = INFINITY;
@@ -171,6 +190,7 @@ __global__ void __launch_bounds__(kPairSuper * kPairChunk) k_pair_prepare(PairSo
       set.ev[chunk] = make_int2(elo, ehi);
       set.lo[chunk] = lo;
       set.hi[chunk] = hi;
+      set.wsum[chunk] = wsum;
     }
   }
   if (lane == 0) ranges[wid] = make_int2(elo, ehi);
@@ -193,11 +213,19 @@ __device__ __forceinline__ float gap(float alo, float ahi, float blo, float bhi)
   return fmaxf(0.f, fmaxf(blo - ahi, alo - bhi));
 }
 
-constexpr int kPairSums = 6;    // s, sz, sq of a lane's two rows
-struct PairSmem {
-  float4 col[3 * kPairChunk];
-  float tot[kPairSums][32];
+// -1 / (2 sigma^2) as the kernels use it: the fast exponent's factor in units
+// of log2, and the exact one's in two parts (both of its sign and not 0, so
+// that an infinite distance stays infinite).
+struct PairScale {
+  float log2, hi, lo;
 };
+
+inline PairScale pair_scale(float sigma) {
+  const double s = 1.0 / (2.0 * (double)sigma * (double)sigma);
+  float hi = (float)s;
+  if ((double)hi > s) hi = nextafterf(hi, 0.f);
+  return PairScale{(float)(-1.4426950408889634074 * s), -hi, -fmaxf((float)(s - (double)hi), 1e-42f)};
+}
 
 // One job of the pair kernel: row tiles of `rows` against `cols`.  With
 // `symmetric` (rows and cols the same set, only the total sum_i w_i s_i
@@ -205,14 +233,23 @@ struct PairSmem {
 struct PairJob {
   PairSet rows, cols;
   float *s, *sz, *sq;       // [slices][rows.n]
+  int32_t *done;            // per tile, for several slices: slices with rows in doubt
   int64_t tiles;
   int slices;
   int symmetric;
 };
 
+constexpr int kPairSums = 6;    // s, sz, sq of the two rows
+struct PairSmem {
+  float4 col[3 * kPairChunk];
+  float tot[kPairSums][32];
+};
+
+// This slice's share of the tile's sums over the columns, in sm.tot; left[]:
+// this lane's part of a bound on what is left out of s, sz and sq.
 template <bool FOUR_D, bool MOMENTS>
-__device__ __forceinline__ void pair_tile(const PairJob &jb, int64_t tile, int slice, float scale, float cut,
-                                          PairSmem &sm, int lane) {
+__device__ __forceinline__ void pair_sums(const PairJob &jb, int64_t tile, int slice, const PairScale &ps, float cut,
+                                          PairSmem &sm, float (&left)[3], int lane) {
   const PairSet &R = jb.rows, &C = jb.cols;
   const int64_t i0 = tile * kPairTile + lane, i1 = i0 + kPairChunk;
   const int64_t nch = (C.n + kPairChunk - 1) / kPairChunk, rch = (R.n + kPairChunk - 1) / kPairChunk;
@@ -228,9 +265,10 @@ __device__ __forceinline__ void pair_tile(const PairJob &jb, int64_t tile, int s
   const float2 X = make_float2(p0.x, p1.x), Y = make_float2(p0.y, p1.y), Z = make_float2(p0.z, p1.z);
   float2 Q = make_float2(0.f, 0.f);
   if (FOUR_D) Q = make_float2(i0 < R.n ? R.q[i0] : 0.f, i1 < R.n ? R.q[i1] : 0.f);
-  const float2 sc = make_float2(scale, scale);
+  const float2 sc = make_float2(ps.log2, ps.log2);
 #pragma unroll
   for (int q = 0; q < kPairSums; ++q) sm.tot[q][lane] = 0.f;
+  left[0] = left[1] = left[2] = 0.f;
   const int64_t first = jb.symmetric ? c0 : 0;
   int turn = 0;
   for (int64_t u0 = (first / kPairSuper) & ~int64_t(31); u0 * kPairSuper < nch; u0 += 32) {
@@ -248,7 +286,14 @@ __device__ __forceinline__ void pair_tile(const PairJob &jb, int64_t tile, int s
           const float4 cl = C.lo[ch], cu = C.hi[ch];
           const float gx = gap(lo.x, hi.x, cl.x, cu.x), gy = gap(lo.y, hi.y, cl.y, cu.y);
           const float gz = gap(lo.z, hi.z, cl.z, cu.z), gq = FOUR_D ? gap(lo.w, hi.w, cl.w, cu.w) : 0.f;
-          near = !((gx * gx + gy * gy + gz * gz + gq * gq) * -scale > cut);
+          const float e = (gx * gx + gy * gy + gz * gz + gq * gq) * -ps.log2;
+          near = !(e > cut);
+          if (!(e > kCutZero)) {
+            const float out = C.wsum[ch] * (near ? kTiny : fmaxf(ex2_approx(-e), kTiny));
+            left[0] += out;
+            if (MOMENTS) left[1] = fmaf(out, fmaxf(hi.z - cl.z, cu.z - lo.z), left[1]);
+            if (MOMENTS && FOUR_D) left[2] = fmaf(out, fmaxf(hi.w - cl.w, cu.w - lo.w), left[2]);
+          }
         }
       }
       unsigned cm = __ballot_sync(0xffffffffu, near);
@@ -309,12 +354,102 @@ __device__ __forceinline__ void pair_tile(const PairJob &jb, int64_t tile, int s
       }
     }
   }
+}
+
+// One row's sums over all columns whose kernel value is not 0 in float32, with
+// expf, by the whole warp; into the first slice's place, zeros into the others.
+// (Few rows: kept out of line.)
+template <bool FOUR_D, bool MOMENTS>
+__device__ __noinline__ void pair_row_exact(const PairJob &jb, int64_t i, const PairScale &ps, int lane) {
+  const PairSet &R = jb.rows, &C = jb.cols;
+  const int64_t nch = (C.n + kPairChunk - 1) / kPairChunk, own = i / kPairTile * 2;   // own: the tile's first chunk
+  const float4 p = R.h[i];
+  const float pq = FOUR_D ? R.q[i] : 0.f;
+  const int2 ev = R.ev[i / kPairChunk];
+  const bool odd = !(isfinite(p.x) && isfinite(p.y) && isfinite(p.z) && isfinite(pq));
+  float acc = 0.f, accz = 0.f, accq = 0.f;
+  for (int64_t cb = jb.symmetric ? own : 0; cb < nch; cb += 32) {
+    const int64_t ch = cb + lane;
+    bool near = false;
+    if (ch < nch) {
+      const int2 r = C.ev[ch];
+      if (r.y >= ev.x && r.x <= ev.y) {
+        const float4 cl = C.lo[ch], cu = C.hi[ch];
+        const float gx = gap(p.x, p.x, cl.x, cu.x), gy = gap(p.y, p.y, cl.y, cu.y), gz = gap(p.z, p.z, cl.z, cu.z);
+        const float gq = FOUR_D ? gap(pq, pq, cl.w, cu.w) : 0.f;
+        near = odd || !((gx * gx + gy * gy + gz * gz + gq * gq) * -ps.log2 > kCutZero);
+      }
+    }
+    for (unsigned m = __ballot_sync(0xffffffffu, near); m; m &= m - 1) {
+      const int64_t k = cb + __ffs(m) - 1, j = k * kPairChunk + lane;
+      const float4 v = C.h[j];
+      const float dx = p.x - v.x, dy = p.y - v.y, dz = p.z - v.z, dq = FOUR_D ? pq - C.q[j] : 0.f;
+      float d = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+      if (FOUR_D) d = fmaf(dq, dq, d);
+      const float kw = expf(fmaf(d, ps.hi, d * ps.lo)) * (jb.symmetric && k > own + 1 ? 2.f * v.w : v.w);
+      acc += kw;
+      if (MOMENTS) accz = fmaf(kw, dz, accz);
+      if (MOMENTS && FOUR_D) accq = fmaf(kw, dq, accq);
+    }
+  }
+  acc = warp_sum(acc);
+  if (MOMENTS) accz = warp_sum(accz);
+  if (MOMENTS && FOUR_D) accq = warp_sum(accq);
+  __syncwarp();            // after the tile's own stores
+  if (lane < jb.slices) {
+    const int64_t o = lane * R.n + i;
+    jb.s[o] = lane == 0 ? acc : 0.f;
+    if (MOMENTS) jb.sz[o] = lane == 0 ? accz : 0.f;
+    if (MOMENTS && FOUR_D) jb.sq[o] = lane == 0 ? accq : 0.f;
+  }
+}
+static_assert(kPairMaxSlices <= 32, "a lane per slice");
+
+template <bool FOUR_D, bool MOMENTS>
+__device__ __forceinline__ void pair_tile(const PairJob &jb, int64_t tile, int slice, const PairScale &ps, float cut,
+                                          PairSmem &sm, int lane) {
+  constexpr int N = MOMENTS ? (FOUR_D ? 3 : 2) : 1;
+  float left[3];
+  pair_sums<FOUR_D, MOMENTS>(jb, tile, slice, ps, cut, sm, left, lane);
 #pragma unroll
-  for (int q = 0; q < 2 * (MOMENTS ? (FOUR_D ? 3 : 2) : 1); ++q) {
+  for (int q = 0; q < 2 * N; ++q) {
     const int64_t i = tile * kPairTile + (q & 1) * kPairChunk + lane;
     float *dst = q < 2 ? jb.s : q < 4 ? jb.sz : jb.sq;
-    if (i < R.n) dst[(int64_t)slice * R.n + i] = sm.tot[q][lane];
+    if (i < jb.rows.n) dst[(int64_t)slice * jb.rows.n + i] = sm.tot[q][lane];
   }
+  // rows in doubt: what is left out may show in their sums' last place
+  auto in_doubt = [&](auto &&sum_of, bool (&unsure)[2]) {
+    unsure[0] = unsure[1] = false;
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+      const float bound = warp_sum(left[q]) * kLeftOut;
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+        if (tile * kPairTile + r * kPairChunk + lane < jb.rows.n)
+          unsure[r] |= !(fabsf(sum_of(q, r)) >= bound);   // (a NaN too)
+    }
+    return __any_sync(0xffffffffu, unsure[0] || unsure[1]);
+  };
+  bool unsure[2];
+  if (!in_doubt([&](int q, int r) { return sm.tot[2 * q + r][lane]; }, unsure)) return;
+  if (jb.slices > 1) {     // none if a slice has none; the last slice looks at the totals
+    __threadfence();
+    __syncwarp();
+    int before = 0;
+    if (lane == 0) before = atomicAdd(jb.done + tile, 1);
+    if (__shfl_sync(0xffffffffu, before, 0) != jb.slices - 1) return;
+    __threadfence();
+    in_doubt([&](int q, int r) {
+      const float *src = (q == 0 ? jb.s : q == 1 ? jb.sz : jb.sq) + tile * kPairTile + r * kPairChunk + lane;
+      float t = 0.f;
+      for (int k = 0; k < jb.slices; ++k) t += __ldcg(src + k * jb.rows.n);
+      return t;
+    }, unsure);
+  }
+#pragma unroll 1
+  for (int r = 0; r < 2; ++r)
+    for (unsigned m = __ballot_sync(0xffffffffu, r ? unsure[1] : unsure[0]); m; m &= m - 1)
+      pair_row_exact<FOUR_D, MOMENTS>(jb, tile * kPairTile + r * kPairChunk + __ffs(m) - 1, ps, lane);
 }
 
 // Up to three jobs in one launch (their warps follow one another, so one
@@ -325,7 +460,7 @@ struct PairJobs {
 };
 
 template <bool FOUR_D>
-__global__ void __launch_bounds__(kPairWarps * 32) k_pair_rows(PairJobs jobs, float scale, float cut) {
+__global__ void __launch_bounds__(kPairWarps * 32) k_pair_rows(PairJobs jobs, PairScale ps, float cut) {
   __shared__ PairSmem sm[kPairWarps];
   const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
   int64_t t = (int64_t)blockIdx.x * kPairWarps + wid;
@@ -336,9 +471,9 @@ __global__ void __launch_bounds__(kPairWarps * 32) k_pair_rows(PairJobs jobs, fl
       const int64_t tile = t / jb.slices;
       const int slice = (int)(t - tile * jb.slices);
       if (jb.sz)
-        pair_tile<FOUR_D, true>(jb, tile, slice, scale, cut, sm[wid], lane);
+        pair_tile<FOUR_D, true>(jb, tile, slice, ps, cut, sm[wid], lane);
       else
-        pair_tile<FOUR_D, false>(jb, tile, slice, scale, cut, sm[wid], lane);
+        pair_tile<FOUR_D, false>(jb, tile, slice, ps, cut, sm[wid], lane);
       return;
     }
     t -= count;
@@ -357,8 +492,8 @@ void launch_pair_rows(const PairJobs &jobs, float sigma, float cut, cudaStream_t
   int64_t warps = 0;
   for (int k = 0; k < jobs.n; ++k) warps += jobs.job[k].tiles * jobs.job[k].slices;
   if (warps <= 0) return;
-  const float scale = (float)(-1.4426950408889634074 / (2.0 * (double)sigma * (double)sigma));
-  k_pair_rows<FOUR_D><<<(unsigned)((warps + kPairWarps - 1) / kPairWarps), kPairWarps * 32, 0, st>>>(jobs, scale, cut);
+  k_pair_rows<FOUR_D><<<(unsigned)((warps + kPairWarps - 1) / kPairWarps), kPairWarps * 32, 0, st>>>(
+      jobs, pair_scale(sigma), cut);
 }
 
 // workspace carving; base null: sizes only
@@ -382,16 +517,17 @@ PairSet take_pair_set(Carver &c, int64_t n, bool four_d) {
   s.ev_up = reinterpret_cast<int2 *>(c.take(sizeof(int2) * (size_t)up));
   s.lo = reinterpret_cast<float4 *>(c.take(sizeof(float4) * (size_t)ch));
   s.hi = reinterpret_cast<float4 *>(c.take(sizeof(float4) * (size_t)ch));
+  s.wsum = c.floats(ch);
   s.n = n;
   return s;
 }
 
 void launch_pair_prepare(const PairSource &sa, const PairSet &a, const PairSource &sb, const PairSet &b,
-                         cudaStream_t st) {
+                         int32_t *done, int64_t n_done, cudaStream_t st) {
   auto blocks = [](int64_t n) { return (pair_chunks(n) + kPairSuper - 1) / kPairSuper; };
   const int64_t ba = blocks(a.n), bb = blocks(b.n);
   if (ba + bb > 0)
-    k_pair_prepare<<<(unsigned)(ba + bb), kPairSuper * kPairChunk, 0, st>>>(sa, a, ba, sb, b);
+    k_pair_prepare<<<(unsigned)(ba + bb), kPairSuper * kPairChunk, 0, st>>>(sa, a, ba, sb, b, done, n_done);
 }
 
 struct MseAdcTotals {
@@ -541,16 +677,23 @@ __global__ void __launch_bounds__(kRedThreads) k_nll_mid(const float *__restrict
   double v[2] = {0, 0};
   const int64_t step = (int64_t)gridDim.x * kRedThreads, at = (int64_t)blockIdx.x * kRedThreads + threadIdx.x;
   for (int64_t i = at; i < n; i += step) v[0] += hp[i];
-  for (int64_t j = at; j < ref.n; j += step) {
-    const float l = slice_sum(lam, ref.n, slices, j) + 1e-10f;
-    const bool on = ref_hp[j] > 0.5f;
+  for (int64_t j0 = at & ~int64_t(31); j0 < ref.n; j0 += step) {   // a warp a chunk
+    const int64_t j = j0 + threadIdx.x % 32;
+    const bool in = j < ref.n;
+    const float l = (in ? slice_sum(lam, ref.n, slices, j) : 0.f) + 1e-10f;
+    const bool on = in && ref_hp[j] > 0.5f;
     const float w = on ? 1.0f / l : 0.0f;
-    ref.h[j].w = w;
+    if (in) ref.h[j].w = w;
     if (on) v[1] += (double)logf(l);
-    if (!isfinite(w)) {   // never passed over by its distance
-      const float inf = INFINITY;
-      ref.lo[j / kPairChunk] = make_float4(-inf, -inf, -inf, -inf);
-      ref.hi[j / kPairChunk] = make_float4(inf, inf, inf, inf);
+    const float wsum = warp_sum(fabsf(w));
+    const bool odd = __any_sync(0xffffffffu, !isfinite(w));
+    if (threadIdx.x % 32 == 0) {
+      ref.wsum[j / kPairChunk] = wsum;
+      if (odd) {   // never passed over by its distance
+        const float inf = INFINITY;
+        ref.lo[j / kPairChunk] = make_float4(-inf, -inf, -inf, -inf);
+        ref.hi[j / kPairChunk] = make_float4(inf, inf, inf, inf);
+      }
     }
   }
   block_sums(v, red, parts + (size_t)blockIdx.x * 2);
@@ -719,6 +862,7 @@ struct MseAdcWs {
   PairSet pred, ref;
   float *a, *az, *b, *bz, *c;
   int slices;      // column slices of every job
+  int32_t *done;   // per tile of the three jobs
   double *parts;
   MseAdcTotals *tot;
 };
@@ -734,6 +878,7 @@ size_t mse_adc_layout(int64_t n, int64_t m, MseAdcWs *w, char *base) {
   s.b = c.floats(n * s.slices);
   s.bz = c.floats(n * s.slices);
   s.c = c.floats(m * s.slices);
+  s.done = reinterpret_cast<int32_t *>(c.floats(2 * pair_tiles(n) + pair_tiles(m)));
   s.parts = reinterpret_cast<double *>(c.take(sizeof(double) * kRedBlocks * kRedMax));
   s.tot = reinterpret_cast<MseAdcTotals *>(c.take(sizeof(MseAdcTotals)));
   if (w) *w = s;
@@ -744,6 +889,7 @@ struct NllWs {
   PairSet pred, ref;
   float *s, *sz, *sq, *lam;
   int slices_p, slices_r;
+  int32_t *done;   // per tile of the two jobs
   double *parts;
 };
 
@@ -758,6 +904,7 @@ size_t nll_layout(int64_t n, int64_t m, NllWs *w, char *base) {
   s.sz = c.floats(n * s.slices_p);
   s.sq = c.floats(n * s.slices_p);
   s.lam = c.floats(m * s.slices_r);
+  s.done = reinterpret_cast<int32_t *>(c.floats(pair_tiles(n) + pair_tiles(m)));
   s.parts = reinterpret_cast<double *>(c.take(sizeof(double) * kRedBlocks * 2));
   if (w) *w = s;
   return c.off;
@@ -779,13 +926,14 @@ int run_mse_adc(const float *x, const float *y, const float *z, const int32_t *e
   MseAdcWs s;
   mse_adc_layout(n, m, &s, static_cast<char *>(ws));
   const HitSet pred{x, y, z, w, event, n}, ref{rx, ry, rz, rw, revent, m};
+  const int64_t tn = pair_tiles(n), tm = pair_tiles(m);
   launch_pair_prepare(PairSource{x, y, z, w, nullptr, event, kEventOffset}, s.pred,
-                      PairSource{rx, ry, rz, rw, nullptr, revent, kEventOffset}, s.ref, st);
+                      PairSource{rx, ry, rz, rw, nullptr, revent, kEventOffset}, s.ref, s.done, 2 * tn + tm, st);
   PairJobs jobs;
   jobs.n = 3;
-  jobs.job[0] = PairJob{s.pred, s.pred, s.a, s.az, nullptr, pair_tiles(n), s.slices, 0};
-  jobs.job[1] = PairJob{s.pred, s.ref, s.b, s.bz, nullptr, pair_tiles(n), s.slices, 0};
-  jobs.job[2] = PairJob{s.ref, s.ref, s.c, nullptr, nullptr, pair_tiles(m), s.slices, 1};
+  jobs.job[0] = PairJob{s.pred, s.pred, s.a, s.az, nullptr, s.done, tn, s.slices, 0};
+  jobs.job[1] = PairJob{s.pred, s.ref, s.b, s.bz, nullptr, s.done + tn, tn, s.slices, 0};
+  jobs.job[2] = PairJob{s.ref, s.ref, s.c, nullptr, nullptr, s.done + 2 * tn, tm, s.slices, 1};
   launch_pair_rows<false>(jobs, sigma, kCutMse, st);
   const unsigned rb = red_blocks(n > m ? n : m);
   k_mse_adc_sums<<<rb, kRedThreads, 0, st>>>(pred, ref, s.a, s.b, s.slices, s.c, s.slices, s.parts);
@@ -806,18 +954,19 @@ int run_nll(const float *x, const float *y, const float *z, const float *q, cons
             cudaStream_t st) {
   NllWs s;
   nll_layout(n, m, &s, static_cast<char *>(ws));
+  const int64_t tn = pair_tiles(n), tm = pair_tiles(m);
   launch_pair_prepare(PairSource{x, y, z, hp, q, event, 1e9f}, s.pred, PairSource{rx, ry, rz, rhp, rq, revent, 1e9f},
-                      s.ref, st);
+                      s.ref, s.done, tn + tm, st);
   PairJobs jobs;
   jobs.n = 1;
   // lambda_j = sum_i hp_i K_ij, then the reference hits weigh 1 / lambda_j
-  jobs.job[0] = PairJob{s.ref, s.pred, s.lam, nullptr, nullptr, pair_tiles(m), s.slices_r, 0};
+  jobs.job[0] = PairJob{s.ref, s.pred, s.lam, nullptr, nullptr, s.done + tn, tm, s.slices_r, 0};
   launch_pair_rows<true>(jobs, sigma, kCutNll, st);
   const unsigned rb = red_blocks(n > m ? n : m);
   k_nll_mid<<<rb, kRedThreads, 0, st>>>(hp, n, rhp, s.lam, s.slices_r, s.ref, s.parts);
   k_nll_reduce<<<1, kRedThreads, 0, st>>>(s.parts, (int)rb, out);
   if (n > 0 && (g_q || g_z || g_hp)) {
-    jobs.job[0] = PairJob{s.pred, s.ref, s.s, s.sz, s.sq, pair_tiles(n), s.slices_p, 0};
+    jobs.job[0] = PairJob{s.pred, s.ref, s.s, s.sz, s.sq, s.done, tn, s.slices_p, 0};
     launch_pair_rows<true>(jobs, sigma, kCutNll, st);
     k_nll_grad<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(hp, n, s.s, s.sz, s.sq, s.slices_p,
                                                             (float)(1.0 / ((double)sigma * (double)sigma)), g_hp,
