@@ -215,13 +215,14 @@ __device__ __forceinline__ float gap(float alo, float ahi, float blo, float bhi)
 
 // -1 / (2 sigma^2) as the kernels use it: the fast exponent's factor in units
 // of log2, and the exact one's in two parts (both of its sign and not 0, so
-// that an infinite distance stays infinite).
+// that an infinite distance stays infinite).  Kept finite, so that hits at the
+// same place have the kernel value 1 however small sigma is.
 struct PairScale {
   float log2, hi, lo;
 };
 
 inline PairScale pair_scale(float sigma) {
-  const double s = 1.0 / (2.0 * (double)sigma * (double)sigma);
+  const double s = fmin(1.0 / (2.0 * (double)sigma * (double)sigma), 2e38);
   float hi = (float)s;
   if ((double)hi > s) hi = nextafterf(hi, 0.f);
   return PairScale{(float)(-1.4426950408889634074 * s), -hi, -fmaxf((float)(s - (double)hi), 1e-42f)};

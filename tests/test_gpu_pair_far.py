@@ -21,7 +21,7 @@ def _grads(fn, a, b, **kw):
 
 def _hits(x, z, w, event=None):
     n = len(x)
-    f = lambda v: np.ascontiguousarray(np.broadcast_to(v, n), np.float32)   # noqa: E731
+    f = lambda v: np.array(np.broadcast_to(v, n), np.float32)   # noqa: E731
     ev = np.zeros(n, np.int32) if event is None else event.astype(np.int32)
     return [f(w), f(x), f(0.0), f(z), f(0.0), f(1.0), ev]
 
@@ -84,3 +84,17 @@ def test_nll_far_hits(cuda, gap, n_near):
     k = np.exp(-0.5 * (dx * dx + dz * dz))
     want = k * dz / (k + 1e-10)
     assert abs(got - want) <= (4 * 0.5 * gap ** 2 + 8) * 2.0 ** -24 * abs(want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sigma", [3e-20, 1e-10, 1e10])
+def test_mse_adc_extreme_sigma(cuda, sigma):
+    """Kernel values 1 at the same place and 0 elsewhere, or 1 everywhere."""
+    w = np.array([1.0, 2.0, 4.0, 8.0], np.float32)
+    a = _hits(np.arange(4.0), np.arange(4.0), w)
+    b = _hits(np.arange(4.0), np.arange(4.0), w[::-1])
+    loss = _grads(losses.mse_adc, a, b, sigma=sigma)[0]
+    same = sigma < 1
+    aa, bb = ((w ** 2).sum(), (w * w[::-1]).sum()) if same else (w.sum() ** 2, w.sum() ** 2)
+    want = 2 * (float(aa) - float(bb)) / float(w.sum()) ** 2
+    assert abs(loss - want) <= 1e-6
