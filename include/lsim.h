@@ -445,9 +445,14 @@ int lsim_pixel_coords(const LsimParams *p, const int32_t *unique_pixels, int64_t
                       int32_t *plane_out, int32_t *event_out, void *stream);
 
 /* Workspace bytes of lsim_fee_prob on the current device, for any number of
- * pixels and paths (one flag per hit step, and the kernel blocks' scratch for
- * path values: about 240 MB at 152 SMs). */
+ * pixels and paths: one flag per hit step, and scratch for the path values of
+ * the pixels that run at the same time (about 240 MB at 152 SMs). */
 size_t lsim_fee_prob_workspace_bytes(const LsimParams *p);
+
+/* The same for calls of at most n_pix pixels, n_t ticks and n_paths paths (of
+ * n_pix beyond two per SM no more is needed): 0.5 MB for one pixel of 2000
+ * ticks at 20 paths. */
+size_t lsim_fee_prob_scratch_bytes(const LsimParams *p, int64_t n_pix, int32_t n_t, int32_t n_paths);
 
 /* Probabilistic self-trigger front end on waveforms wfs[n_pix][n_t]
  * (n_t <= 2048): the beam search over n_paths (fee_paths_scaling <= 32)

@@ -394,7 +394,11 @@ int lsim_pixel_coords(const LsimParams *p, const int32_t *unique_pixels, int64_t
 }
 
 size_t lsim_fee_prob_workspace_bytes(const LsimParams *p) {
-  return p ? fee_prob_workspace_bytes(p->max_adc_values) : 0;
+  return p ? fee_prob_workspace_bytes() : 0;
+}
+
+size_t lsim_fee_prob_scratch_bytes(const LsimParams *p, int64_t n_pix, int32_t n_t, int32_t n_paths) {
+  return p && n_pix >= 0 ? fee_prob_workspace_bytes(n_pix, n_t, n_paths) : 0;
 }
 
 static int fee_prob(const LsimParams *p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
@@ -406,9 +410,9 @@ static int fee_prob(const LsimParams *p, const float *wfs, int64_t n_pix, int32_
   if (any_red && !(exp_tick_out && exp_adc_out && lambda_out))
     return fail(LSIM_ERR_INVALID, "%s: give all three of exp_tick, exp_adc, lambda or none", name);
   if (!(stop_threshold > 0.0f)) return fail(LSIM_ERR_INVALID, "%s: stop_threshold %g", name, stop_threshold);
-  if (!ws || ws_bytes < fee_prob_workspace_bytes(p->max_adc_values))
-    return fail(LSIM_ERR_CAPACITY, "%s: workspace %zu < %zu bytes", name, ws_bytes,
-                fee_prob_workspace_bytes(p->max_adc_values));
+  const size_t need = fee_prob_workspace_bytes(n_pix, n_t, n_paths);
+  if (!ws || ws_bytes < need)
+    return fail(LSIM_ERR_CAPACITY, "%s: workspace %zu < %zu bytes", name, ws_bytes, need);
   return wrap(run_fee_prob(*p, wfs, n_pix, n_t, n_paths, stop_threshold, log_prob_out, charge_out, exp_tick_out,
                            exp_adc_out, lambda_out, record, ws, (cudaStream_t)stream),
               name);

@@ -208,7 +208,8 @@ struct ProbArgs {
   float *log_prob, *charge, *e_tick, *e_adc, *lam;
   unsigned long long *work;   // pixels handed out beyond the blocks' first
   int32_t *step_active;   // [H]: some pixel kept a total path probability above the stop level after step h
-  float *cache;           // [blocks][K][kCacheArrays][kProbMaxT]: path values kept from step to step
+  float *cache;           // [blocks][K][kCacheArrays][cache_row]: path values kept from step to step
+  int cache_row;          // floats per row of the cache, at least T - 1
   bool all_steps;         // run every step even when nothing can come of it
   // record for the adjoint (all or none):
   float *state;           // [n_pix][H][2][K]: each step's input path charges and log-probabilities
@@ -241,9 +242,12 @@ constexpr float kWeakRise = 1.4f, kWeakMost = -190.0f;
 // enters the log-sum-exps), and two thirds of a pixel's paths carry a charge
 // that a path of the step before carried (after the last real hit the top-K
 // ticks hardly change).  So the values of a path are kept in the block's
-// scratch (global memory, in L2) for as long as some path has its charge:
-// a step evaluates new charges only and then folds the K paths' kept values,
-// in the order and with the operations of an evaluation in place.
+// scratch for as long as some path has its charge: a step evaluates new
+// charges only and then folds the K paths' kept values, in the order and with
+// the operations of an evaluation in place.  The scratch is global memory:
+// the values-only form uses 10 to 30 % of it, which stays in L2; with the
+// distributions of dense 2000-tick rows it is 20 x 3 x 2000 floats a block,
+// 146 MB over 304 blocks, and does not fit in the 129 MB.
 //
 // Without the distributions (kDist false) a value matters only where its
 // probability does not underflow, and the rest is left out exactly:
@@ -288,8 +292,8 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob(ProbArgs a) {
   const float z = a.z, thr = a.thr;
   const float term_m1 = ldn_log_term(-1.0f);
   const float log_k = logf((float)K) + 1e-3f;
-  float *cache = a.cache + (size_t)blockIdx.x * K * kCacheArrays * kProbMaxT;
-  auto kept = [&](int slot, int what) { return cache + (size_t)(slot * kCacheArrays + what) * kProbMaxT; };
+  float *cache = a.cache + (size_t)blockIdx.x * K * kCacheArrays * a.cache_row;
+  auto kept = [&](int slot, int what) { return cache + (size_t)(slot * kCacheArrays + what) * a.cache_row; };
   auto shifted = [&](int t) { return min(t + a.interval + 1, T - 1); };
   // the hit term of a path at tick t from its two log_ndtr values and its dist term
   auto hit_term = [&](int t, float zqs, float zq0, float LQs, float LQ0, float lg) {
@@ -1217,10 +1221,16 @@ static unsigned long long *work_counter(int32_t *flags) {
   return reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(flags) + kFlagBytes) - 1;
 }
 
-// step_active, then the blocks' path values (for any number of paths and pixels)
-size_t fee_prob_workspace_bytes(int32_t) {
-  return kFlagBytes + sizeof(float) * (size_t)prob_blocks() * kProbMaxPaths * kCacheArrays * kProbMaxT;
+static int cache_row(int32_t n_t) { return n_t < 32 ? 32 : n_t > kProbMaxT ? kProbMaxT : (n_t + 31) & ~31; }
+
+// step_active, then the path values of the blocks that a call starts
+size_t fee_prob_workspace_bytes(int64_t n_pix, int32_t n_t, int32_t n_paths) {
+  const int64_t cap = prob_blocks(), blocks = n_pix < 0 ? 0 : n_pix < cap ? n_pix : cap;
+  const int paths = n_paths < 1 ? 1 : n_paths > kProbMaxPaths ? kProbMaxPaths : n_paths;
+  return al256(kFlagBytes + sizeof(float) * (size_t)blocks * paths * kCacheArrays * cache_row(n_t));
 }
+
+size_t fee_prob_workspace_bytes() { return fee_prob_workspace_bytes(INT64_MAX, kProbMaxT, kProbMaxPaths); }
 
 struct ProbRecord {
   int32_t *step_active, *n_run, *top;
@@ -1302,6 +1312,7 @@ static int run_fee_prob_impl(const LsimParams &p, const float *wfs, int64_t n_pi
   char *b = static_cast<char *>(ws);
   a.step_active = reinterpret_cast<int32_t *>(b);
   a.cache = reinterpret_cast<float *>(b + kFlagBytes);
+  a.cache_row = cache_row(n_t);
   if (record) {
     ProbRecord r;
     record_layout(n_pix, p.max_adc_values, n_paths, &r, static_cast<char *>(record));
@@ -1358,7 +1369,7 @@ int run_fee_prob_vjp_recorded(const LsimParams &p, const float *wfs, int64_t n_p
 }
 
 size_t fee_prob_vjp_workspace_bytes(int64_t n_pix, int32_t max_adc_values, int32_t n_paths) {
-  return fee_prob_workspace_bytes(max_adc_values) + fee_prob_record_bytes(n_pix, max_adc_values, n_paths);
+  return fee_prob_workspace_bytes(n_pix, kProbMaxT, n_paths) + fee_prob_record_bytes(n_pix, max_adc_values, n_paths);
 }
 
 int run_fee_prob_vjp(const LsimParams &p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,

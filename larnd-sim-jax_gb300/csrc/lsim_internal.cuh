@@ -68,7 +68,8 @@ int run_pixel_coords(const LsimParams &p, const int32_t *unique_pixels, int64_t 
                      int32_t *plane, int32_t *event, cudaStream_t st);
 
 // lsim_fee_prob.cu
-size_t fee_prob_workspace_bytes(int32_t max_adc_values);
+size_t fee_prob_workspace_bytes();   // for any call
+size_t fee_prob_workspace_bytes(int64_t n_pix, int32_t n_t, int32_t n_paths);
 int run_fee_prob(const LsimParams &p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
                  float stop_threshold, float *log_prob, float *charge, float *e_tick, float *e_adc, float *lam,
                  void *record, void *ws, cudaStream_t st);

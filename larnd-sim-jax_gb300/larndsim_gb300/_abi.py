@@ -119,6 +119,7 @@ _SIGNATURES = {
                                     _vp]),
     "lsim_pixel_coords": (C.c_int, [_PP, _vp, _i64, _vp, _vp, _vp, _vp, _vp]),
     "lsim_fee_prob_workspace_bytes": (_sz, [_PP]),
+    "lsim_fee_prob_scratch_bytes": (_sz, [_PP, _i64, _i32, _i32]),
     "lsim_fee_prob": (C.c_int, [_PP, _vp, _i64, _i32, _i32, C.c_float, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
     "lsim_fee_prob_record_bytes": (_sz, [_PP, _i64, _i32]),
     "lsim_fee_prob_record": (C.c_int, [_PP, _vp, _i64, _i32, _i32, C.c_float, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp,

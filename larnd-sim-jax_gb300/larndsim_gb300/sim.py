@@ -363,7 +363,7 @@ def _fee_prob(params, wfs, stop_threshold, distributions, reductions, record=Fal
     H = int(params.MAX_ADC_VALUES)
     K = int(params.fee_paths_scaling)
     lp = _abi.make_params(params)
-    ws = torch.empty(lib.lsim_fee_prob_workspace_bytes(lp), dtype=torch.uint8, device=w.device)
+    ws = torch.empty(lib.lsim_fee_prob_scratch_bytes(lp, P, T, K), dtype=torch.uint8, device=w.device)
     f = dict(dtype=torch.float32, device=w.device)
     log_prob = torch.empty((P, H, T - 1), **f) if distributions else None
     charge = torch.empty((P, H, T - 1), **f) if distributions else None
