@@ -482,7 +482,9 @@ int lsim_fee_prob_record(const LsimParams *p, const float *wfs, int64_t n_pix, i
 /* Vector-Jacobian product as lsim_fee_prob_vjp, on the record of a forward on
  * the same waveforms instead of a re-run.  A cotangent on the
  * log-probabilities or charges needs a record made with log_prob_out or
- * charge_out. */
+ * charge_out.  With a record that lacks it, or of another n_pix, n_t, n_paths
+ * or MAX_ADC_VALUES, g_wfs is filled with NaN (the record is device memory
+ * that the forward may still be writing, so the call returns LSIM_OK). */
 int lsim_fee_prob_vjp_recorded(const LsimParams *p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
                                const void *record, size_t record_bytes, const float *g_log_prob,
                                const float *g_charge, const float *g_e_tick, const float *g_e_adc,

@@ -199,6 +199,14 @@ __device__ __forceinline__ float block_sum(float v, float *red) {
   return t;
 }
 
+// What a record was made from, kept with it: the adjoint compares it with its
+// own call (on the device: the host does not wait for the forward).
+struct ProbMark {
+  int64_t n_pix;
+  int32_t T, K, H;
+  int32_t all_steps;      // every tick, path and step is in it: serves cotangents on the distributions
+};
+
 struct ProbArgs {
   LsimParams p;
   const float *wfs;
@@ -212,6 +220,7 @@ struct ProbArgs {
   int cache_row;          // floats per row of the cache, at least T - 1
   bool all_steps;         // run every step even when nothing can come of it
   // record for the adjoint (all or none):
+  ProbMark *mark;
   float *state;           // [n_pix][H][2][K]: each step's input path charges and log-probabilities
   int32_t *state_top;     // [n_pix][H][K]: each step's selected ticks
   uint32_t *live;         // [n_pix][H][kLiveWords]: ticks whose probability is not 0
@@ -304,6 +313,7 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob(ProbArgs a) {
   };
 
   bool leave_out = !kDist && !a.all_steps;
+  if (a.mark && blockIdx.x == 0 && tid == 0) *a.mark = ProbMark{a.n_pix, T, K, H, leave_out ? 0 : 1};
   for (int64_t pix = blockIdx.x; pix < a.n_pix;) {
     const float *w = a.wfs + pix * T;
     for (int t = tid; t < T; t += kProbThreads) qs[t] = w[t] * p.t_sampling;
@@ -802,7 +812,7 @@ struct LogDiff {
 };
 
 struct ProbVjpArgs {
-  ProbArgs f;                  // the forward's arguments (its record, step_active and reductions read)
+  ProbArgs f;                  // the forward's arguments (its record, mark, step_active and reductions read)
   const float *g_log_prob;     // optional [n_pix][H][T-1]
   const float *g_charge;       // optional [n_pix][H][T-1]
   const float *g_e_tick, *g_e_adc, *g_lam;   // optional [n_pix][H] (all three or none)
@@ -879,6 +889,15 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
   }
   __syncthreads();
 
+  // a record of another call, or one that leaves out what a cotangent on the
+  // distributions needs, has no gradient to give (its ticks may not even fit)
+  const ProbMark mk = *a.mark;
+  if (mk.n_pix != a.n_pix || mk.T != T || mk.K != K || mk.H != H ||
+      ((va.g_log_prob || va.g_charge) && !mk.all_steps)) {
+    for (int64_t pix = blockIdx.x; pix < a.n_pix; pix += gridDim.x)
+      for (int t = tid; t < T; t += kProbThreads) va.g_wfs[pix * T + t] = NAN;
+    return;
+  }
   // the record is only read here: backward passes may share it
   for (int64_t pix = blockIdx.x; pix < a.n_pix; pix += gridDim.x) {
     const float *w = a.wfs + pix * T;
@@ -1214,9 +1233,10 @@ static int64_t prob_blocks() { return (int64_t)device_sm_count() * 2; }
 
 static size_t al256(size_t b) { return (b + 255) & ~size_t(255); }
 
-// The steps' flags and, at the end of their 256 bytes, the forward's pixel counter.
-constexpr size_t kFlagBytes = 256;
-static_assert(sizeof(int32_t) * LSIM_MAX_HITS + sizeof(unsigned long long) <= kFlagBytes, "flags and counter");
+// The steps' flags, a record's mark and, at the end of their 256 bytes, the forward's pixel counter.
+constexpr size_t kFlagBytes = 256, kMarkAt = 64;
+static_assert(sizeof(int32_t) * LSIM_MAX_HITS <= kMarkAt && kMarkAt % alignof(ProbMark) == 0 &&
+              kMarkAt + sizeof(ProbMark) + sizeof(unsigned long long) <= kFlagBytes, "flags, mark and counter");
 static unsigned long long *work_counter(int32_t *flags) {
   return reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(flags) + kFlagBytes) - 1;
 }
@@ -1233,6 +1253,7 @@ size_t fee_prob_workspace_bytes(int64_t n_pix, int32_t n_t, int32_t n_paths) {
 size_t fee_prob_workspace_bytes() { return fee_prob_workspace_bytes(INT64_MAX, kProbMaxT, kProbMaxPaths); }
 
 struct ProbRecord {
+  ProbMark *mark;
   int32_t *step_active, *n_run, *top;
   float *state, *red;
   uint32_t *live;
@@ -1253,7 +1274,7 @@ static size_t record_layout(int64_t n_pix, int32_t max_adc_values, int32_t n_pat
   char *live = take(sizeof(uint32_t) * steps * kLiveWords);
   char *red = take(sizeof(float) * 3 * steps);
   if (r)
-    *r = ProbRecord{reinterpret_cast<int32_t *>(active), reinterpret_cast<int32_t *>(run),
+    *r = ProbRecord{reinterpret_cast<ProbMark *>(active + kMarkAt), reinterpret_cast<int32_t *>(active), reinterpret_cast<int32_t *>(run),
                     reinterpret_cast<int32_t *>(top), reinterpret_cast<float *>(state),
                     reinterpret_cast<float *>(red), reinterpret_cast<uint32_t *>(live)};
   return off;
@@ -1316,6 +1337,7 @@ static int run_fee_prob_impl(const LsimParams &p, const float *wfs, int64_t n_pi
   if (record) {
     ProbRecord r;
     record_layout(n_pix, p.max_adc_values, n_paths, &r, static_cast<char *>(record));
+    a.mark = r.mark;
     a.step_active = r.step_active;
     a.state = r.state;
     a.state_top = r.top;
@@ -1343,6 +1365,7 @@ int run_fee_prob_vjp_recorded(const LsimParams &p, const float *wfs, int64_t n_p
   record_layout(n_pix, p.max_adc_values, n_paths, &r, const_cast<char *>(static_cast<const char *>(record)));
   ProbVjpArgs va{};
   va.f = prob_args(p, wfs, n_pix, n_t, n_paths);
+  va.f.mark = r.mark;
   va.f.step_active = r.step_active;
   va.f.state = r.state;
   va.f.state_top = r.top;
