@@ -394,10 +394,15 @@ def _fee_prob_vjp(params, wfs, rec, g_lp=None, g_ch=None, g_red=None):
     return g
 
 
+# grad_mode: torch.is_grad_enabled() of the caller (inside forward it is always
+# off, and needs_input_grad tells of the input alone): without it no backward
+# pass can follow and no record is made.
+
 class _FeeProbDistFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, wfs, params, stop_threshold):
-        log_prob, charge, _, rec = _fee_prob(params, wfs, stop_threshold, True, False, ctx.needs_input_grad[0])
+    def forward(ctx, wfs, params, stop_threshold, grad_mode):
+        log_prob, charge, _, rec = _fee_prob(params, wfs, stop_threshold, True, False,
+                                             grad_mode and ctx.needs_input_grad[0])
         ctx.save_for_backward(wfs, rec)
         ctx.params = params
         return log_prob, charge
@@ -405,13 +410,14 @@ class _FeeProbDistFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g_lp, g_ch):
         wfs, rec = ctx.saved_tensors
-        return _fee_prob_vjp(ctx.params, wfs, rec, g_lp=g_lp, g_ch=g_ch), None, None
+        return _fee_prob_vjp(ctx.params, wfs, rec, g_lp=g_lp, g_ch=g_ch), None, None, None
 
 
 class _FeeProbRedFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, wfs, params, stop_threshold):
-        _, _, (e_tick, e_adc, lam), rec = _fee_prob(params, wfs, stop_threshold, False, True, ctx.needs_input_grad[0])
+    def forward(ctx, wfs, params, stop_threshold, grad_mode):
+        _, _, (e_tick, e_adc, lam), rec = _fee_prob(params, wfs, stop_threshold, False, True,
+                                                    grad_mode and ctx.needs_input_grad[0])
         ctx.save_for_backward(wfs, rec)
         ctx.params = params
         return e_tick, e_adc, lam
@@ -421,7 +427,7 @@ class _FeeProbRedFn(torch.autograd.Function):
         wfs, rec = ctx.saved_tensors
         zero = lambda g: torch.zeros(wfs.shape[0], int(ctx.params.MAX_ADC_VALUES), device=wfs.device) \
             if g is None else g   # noqa: E731
-        return _fee_prob_vjp(ctx.params, wfs, rec, g_red=(zero(g_t), zero(g_a), zero(g_l))), None, None
+        return _fee_prob_vjp(ctx.params, wfs, rec, g_red=(zero(g_t), zero(g_a), zero(g_l))), None, None, None
 
 
 def _as_wfs(wfs):
@@ -436,7 +442,7 @@ def get_adc_values_average_noise_vmap(params, wfs, stop_threshold=1e-9):
     (P, MAX_ADC_VALUES, T - 1): the log-probability that hit h is read at
     each tick and the expected charge if it is.  Differentiable with
     respect to ``wfs`` (lsim_fee_prob_vjp)."""
-    return _FeeProbDistFn.apply(_as_wfs(wfs), params, stop_threshold)
+    return _FeeProbDistFn.apply(_as_wfs(wfs), params, stop_threshold, torch.is_grad_enabled())
 
 
 def average_hit_values(params, wfs, stop_threshold=1e-9):
@@ -445,7 +451,7 @@ def average_hit_values(params, wfs, stop_threshold=1e-9):
     distributions are never stored: (expected_ticks, expected_adcs,
     lambda), each (P, MAX_ADC_VALUES).  Differentiable with respect to
     ``wfs`` (lsim_fee_prob_vjp)."""
-    return _FeeProbRedFn.apply(_as_wfs(wfs), params, stop_threshold)
+    return _FeeProbRedFn.apply(_as_wfs(wfs), params, stop_threshold, torch.is_grad_enabled())
 
 
 def get_average_hit_values(ticks_prob, adcs_distrib):
