@@ -878,6 +878,10 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
   // the esperance and the soft-where weight of tick t, recomputed from q
   auto esp_at = [&](int t) { return (qs[shifted(t)] + thr) - 0.5f * (qs[t + 1] + qs[t]); };
   auto sw_at = [&](float e) { return sigmoid_f((e - thr) * 10.0f); };
+  // whether every tick's cotangent from the reductions' is finite
+  auto finite_cotangents = [&](float gl, float gt, float ga, float den) {
+    return isfinite(fabsf(gl) + fabsf(gt) * (float)T / den + fabsf(ga) * p.adc_counts / den);
+  };
   if (tid == 0) {
     int first = H;
     for (int h = 1; h < H; ++h)
@@ -937,7 +941,20 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
     const int U = n_cls;
     if (tid == 0) rep[U] = (uint16_t)(T - 1);     // end of the last class
 
-    for (int h = min(n_exec, a.n_run[pix]) - 1; h >= 0; --h) {
+    const int n_run = min(n_exec, a.n_run[pix]);
+    if (va.g_lam && n_run < n_exec) {
+      // steps left out, every probability of theirs 0: a cotangent that is not finite is NaN on every tick
+      bool odd = false;
+      for (int h = n_run + tid; h < n_exec; h += kProbThreads) {
+        const int64_t o = pix * H + h;
+        odd |= !finite_cotangents(va.g_lam[o], va.g_e_tick[o], va.g_e_adc[o], 1e-10f);
+      }
+      if (__syncthreads_or(odd)) {
+        for (int t = tid; t < T; t += kProbThreads) va.g_wfs[pix * T + t] = NAN;
+        continue;
+      }
+    }
+    for (int h = n_run - 1; h >= 0; --h) {
       const int64_t o = pix * H + h;
       // step h's input paths and selected ticks, recorded by the forward
       if (tid < K) {
@@ -983,6 +1000,19 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
       if (va.g_charge)
         for (int t = tid; t < T - 1; t += kProbThreads) Aesp[t] += va.g_charge[o * (int64_t)(T - 1) + t];
       __syncthreads();
+      // the reductions' cotangents, common to the step's ticks
+      float gl = 0.f, gt = 0.f, ga = 0.f, den = 1.f;
+      bool odd = false;      // not finite: a tick without probability has a cotangent too (0 times infinity)
+      if (va.g_lam) {
+        const float ET = a.red[o], EA = a.red[a.n_pix * H + o], L = a.red[2 * a.n_pix * H + o];
+        den = fmaxf(L, 1e-10f);
+        const float on = L > 1e-10f ? 1.f : (L == 1e-10f ? 0.5f : 0.f);   // jnp.maximum's share
+        gt = va.g_e_tick[o];
+        ga = va.g_e_adc[o];
+        // the lambda cotangent also reaches ET and EA through the denominator
+        gl = va.g_lam[o] + on * (-(gt * ET + ga * EA) / den);
+        odd = !finite_cotangents(gl, gt, ga, den);
+      }
       // ---- the classes with a cotangent, in order
       unsigned live_bits[kProbTicks];
 #pragma unroll
@@ -991,7 +1021,7 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
         bool live = false;
         if (u < U) {
           const int t = rep[u];
-          live = tmp[u] != 0.f;
+          live = odd || tmp[u] != 0.f;
           if (va.g_lam && !live) live = (a.live[o * kLiveWords + (t >> 5)] >> (t & 31)) & 1u;
           if (va.g_log_prob)
             for (int tt = t; tt < rep[u + 1] && !live; ++tt) live = va.g_log_prob[o * (int64_t)(T - 1) + tt] != 0.f;
@@ -1022,17 +1052,6 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
         }
       }
       __syncthreads();
-      // the reductions' cotangents, common to the step's ticks
-      float gl = 0.f, gt = 0.f, ga = 0.f, den = 1.f;
-      if (va.g_lam) {
-        const float ET = a.red[o], EA = a.red[a.n_pix * H + o], L = a.red[2 * a.n_pix * H + o];
-        den = fmaxf(L, 1e-10f);
-        const float on = L > 1e-10f ? 1.f : (L == 1e-10f ? 0.5f : 0.f);   // jnp.maximum's share
-        gt = va.g_e_tick[o];
-        ga = va.g_e_adc[o];
-        // the lambda cotangent also reaches ET and EA through the denominator
-        gl = va.g_lam[o] + on * (-(gt * ET + ga * EA) / den);
-      }
       auto at = [&](int what, int i) -> float & { return pair[what * kPairStride + i]; };
       const int na = n_act, per_round = kProbThreads / na;   // classes per round of pairs
       const int my = tid / na;                                // this thread's class in a round

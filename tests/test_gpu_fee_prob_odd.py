@@ -1,0 +1,68 @@
+"""Adjoint of the probabilistic front end with cotangents and rows that are not
+finite: a NaN or an infinity on any hit of a row makes the row's gradient NaN
+(0 probability times infinity included) and touches no other row."""
+
+import numpy as np
+import pytest
+
+from larndsim_gb300 import consts, sim
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows(n, T):
+    import torch
+    rng = np.random.default_rng(T)
+    w = np.zeros((n, T), np.float32)
+    for r in range(n):
+        t = rng.integers(T // 8, T // 2)
+        w[r, t:t + T // 8] = rng.uniform(500, 3000)
+    w[0, T // 16:-T // 16] = 3000      # hits on every step, so that no step is left out for the batch
+    return torch.from_numpy(w).cuda()
+
+
+def _grad(w, cot):
+    import torch
+    w = w.detach().requires_grad_(True)
+    out = sim.average_hit_values(consts.Params(), w)
+    torch.autograd.backward(out, cot)
+    return w.grad, out
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf, 3e38])
+@pytest.mark.parametrize("which", [0, 1, 2])
+@pytest.mark.parametrize("hit", [0, 1, 9])
+def test_odd_cotangent(cuda, hit, which, value):
+    """On the first hit, on one without probability and on the last step; 3e38
+    overflows over the smallest denominator, 1e-10, of a hit without probability."""
+    import torch
+    n, T, H = 6, 700, 10
+    w = _rows(n, T)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    cot = [torch.randn((n, H), generator=g, device="cuda") for _ in range(3)]
+    clean, out = _grad(w, cot)
+    lam = out[2].detach()
+    assert float(lam[0].min()) > 0.5 and float(lam[2, 9]) == 0
+    if np.isfinite(value) and (which == 2 or float(lam[2, hit]) > 0):
+        pytest.skip("finite on a hit with a probability")
+    cot[which][2, hit] = value
+    got, _ = _grad(w, cot)
+    keep = [r for r in range(n) if r != 2]
+    assert torch.equal(got[keep], clean[keep])
+    assert bool(torch.isnan(got[2]).all())
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_odd_row(cuda, value):
+    import torch
+    n, T, H = 6, 700, 10
+    w = _rows(n, T)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    cot = [torch.randn((n, H), generator=g, device="cuda") for _ in range(3)]
+    clean, _ = _grad(w, cot)
+    odd = w.clone()
+    odd[3, 400] = value
+    got, out = _grad(odd, cot)
+    keep = [r for r in range(n) if r != 3]
+    assert torch.equal(got[keep], clean[keep])
+    assert bool(torch.isnan(out[1][3].detach()).any()) and bool(torch.isnan(got[3]).all())
