@@ -280,7 +280,11 @@ def make_params(params, lut_shape=None) -> LsimParams:
     lp.nb_bins_per_pixel = nb
     lp.n_tran_bins = int(params.nb_tran_diff_bins)
     lp.n_neighbors = int(params.number_pix_neighbors)
-    edges = _tran_edges(int(params.nb_tran_diff_bins), float(params.pixel_pitch), float(nb))[:8]
+    n, pitch, bins = params.nb_tran_diff_bins, params.pixel_pitch, params.nb_sampling_bins_per_pixel
+    if type(n) is int and type(pitch) is float and type(bins) is int:
+        edges = _tran_edges(n, pitch, bins)[:8]
+    else:           # other types round in their own arithmetic
+        edges = consts.tran_diff_edges(n, pitch, bins)[:8].tolist()
     lp.tran_edges[:len(edges)] = edges
     lp.t_sampling = float(params.t_sampling)
     lp.n_ticks = consts.n_ticks(params)
