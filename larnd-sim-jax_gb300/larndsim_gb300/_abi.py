@@ -245,7 +245,34 @@ def _tran_edges(nb, pitch, bins):
     return tuple(consts.tran_diff_edges(nb, pitch, bins).tolist())
 
 
+# Parameters that stand alone in the block, so that one that the caller's mode
+# does not use may be None (NaN in the block).
+_MAY_BE_UNSET = frozenset(("Ab", "kb", "alpha", "beta", "MeVToElectrons", "lifetime", "long_diff", "tran_diff",
+                           "size_margin", "shift_x", "shift_y", "shift_z", "DISCRIMINATION_THRESHOLD", "GAIN",
+                           "V_PEDESTAL", "ADC_COUNTS", "RESET_NOISE_CHARGE", "UNCORRELATED_NOISE_CHARGE",
+                           "hit_prob_threshold"))
+
+
+class _UnsetAsNan:
+    def __init__(self, params):
+        self._params = params
+
+    def __getattr__(self, name):
+        v = getattr(self._params, name)
+        return float("nan") if v is None and name in _MAY_BE_UNSET else v
+
+
 def make_params(params, lut_shape=None) -> LsimParams:
+    """The LsimParams block of a Params object (_fill_params)."""
+    try:
+        return _fill_params(params, lut_shape)
+    except TypeError:
+        if all(getattr(params, k) is not None for k in _MAY_BE_UNSET):
+            raise
+        return _fill_params(_UnsetAsNan(params), lut_shape)
+
+
+def _fill_params(params, lut_shape) -> LsimParams:
     """Fill an LsimParams block from a Params object.
 
     ``lut_shape`` = (n_templates, nx, ny, nt) of the template bank (LUT

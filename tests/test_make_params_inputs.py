@@ -1,9 +1,19 @@
 """make_params on parameter values that are not plain numbers."""
 
+import math
+
 import numpy as np
 import pytest
 
 from larndsim_gb300 import _abi, consts
+
+
+@pytest.mark.parametrize("field", ["Ab", "kb", "alpha", "beta", "shift_x", "UNCORRELATED_NOISE_CHARGE"])
+def test_unset_parameter_is_nan(field):
+    """A parameter that the recombination mode or the path does not use may be None."""
+    lp = _abi.make_params(consts.Params(**{field: None}))
+    name = {"UNCORRELATED_NOISE_CHARGE": "uncorr_noise"}.get(field, field)
+    assert math.isnan(getattr(lp, name))
 
 
 @pytest.mark.parametrize("pitch", [np.float32(0.38), np.float32(0.4434), np.float64(0.38), np.array(0.38, np.float32)])
