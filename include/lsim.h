@@ -116,7 +116,7 @@ void lsim_struct_sizes(size_t *params, size_t *fields, size_t *counts);
  * calls.  Not part of the reference interface. */
 typedef struct LsimTuning {
   int32_t pixel_blocks_per_sm;  /* persistent pixel-kernel blocks per SM, 1..occupancy limit */
-  int32_t main_blocks;          /* blocks of the segment-major main-bin kernels */
+  int32_t main_blocks;          /* blocks of the segment-major main-bin kernels (at most 65536 are launched) */
   int32_t main_block_warps;     /* warps per main-bin block: 8 or 4 (other values: the default, 24) */
   int32_t reserved[5];
 } LsimTuning;

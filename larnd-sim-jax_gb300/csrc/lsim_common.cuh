@@ -155,7 +155,6 @@ struct Workspace {
 
 constexpr int kPixRec = 12;      // floats per per-pixel record (loss + 8 grads, padded)
 constexpr int kRedSlots = 4096;  // reduction blocks (pixels + main-bin warps + target-only)
-constexpr int kMainWarps = 8192; // warps of the segment-major main-bin kernels
 constexpr int kMaxTemplates = 1024;    // long-diffusion templates the main-bin ordering supports
 constexpr int kMainRecPerSeg = 4;      // a segment's main bins cover at most 2 x 2 pixels
 constexpr int kMainRecFloats = 164;    // window of 160 samples + d(corr)/d(frac), padded to 16 bytes

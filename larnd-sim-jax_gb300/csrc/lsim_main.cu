@@ -175,12 +175,13 @@ __device__ __forceinline__ void slot_offset(const SegFwd &f, int slot, int *dx, 
 // 1.25 and 1.46.  Measured there: 16 warps a block 1.37-1.65 / 1.60-1.91,
 // 32 warps 1.31-1.35 / 1.53-1.56, segments per warp 1, 3, 4: 1.31, 1.43, 1.39.
 constexpr int kMainSmWarps = 24;
+constexpr int kMaxMainBlocks = 65536;    // of a tuned shape: more blocks than segments only cost their launch
 
 template <typename F>
 static void with_main_shape(F &&launch) {
   const LsimTuning tu = tuning();
   const int warps = tu.main_block_warps == 8 || tu.main_block_warps == 4 ? tu.main_block_warps : kMainSmWarps;
-  const int blocks = tu.main_blocks > 0 ? min(tu.main_blocks, kMainWarps / warps)
+  const int blocks = tu.main_blocks > 0 ? min(tu.main_blocks, kMaxMainBlocks)
                                         : device_sm_count() * (kMainSmWarps / warps);
   if (warps == 4) launch(std::integral_constant<int, 4>(), blocks);
   else if (warps == 8) launch(std::integral_constant<int, 8>(), blocks);
