@@ -1003,6 +1003,7 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
       // the reductions' cotangents, common to the step's ticks
       float gl = 0.f, gt = 0.f, ga = 0.f, den = 1.f;
       bool odd = false;      // not finite: a tick without probability has a cotangent too (0 times infinity)
+      bool none = true;      // all zero: no tick has a cotangent from them
       if (va.g_lam) {
         const float ET = a.red[o], EA = a.red[a.n_pix * H + o], L = a.red[2 * a.n_pix * H + o];
         den = fmaxf(L, 1e-10f);
@@ -1012,6 +1013,7 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
         // the lambda cotangent also reaches ET and EA through the denominator
         gl = va.g_lam[o] + on * (-(gt * ET + ga * EA) / den);
         odd = !finite_cotangents(gl, gt, ga, den);
+        none = gl == 0.f && gt == 0.f && ga == 0.f;
       }
       // ---- the classes with a cotangent, in order
       unsigned live_bits[kProbTicks];
@@ -1022,7 +1024,7 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
         if (u < U) {
           const int t = rep[u];
           live = odd || tmp[u] != 0.f;
-          if (va.g_lam && !live) live = (a.live[o * kLiveWords + (t >> 5)] >> (t & 31)) & 1u;
+          if (!none && !live) live = (a.live[o * kLiveWords + (t >> 5)] >> (t & 31)) & 1u;
           if (va.g_log_prob)
             for (int tt = t; tt < rep[u + 1] && !live; ++tt) live = va.g_log_prob[o * (int64_t)(T - 1) + tt] != 0.f;
         }
@@ -1073,10 +1075,10 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
           const float LQ0 = log_ndtr_f(zq0), LQs = log_ndtr_f(zqs);
           const LogDiff dq(zqs, zq0, LQs, LQ0, term_m1);
           const float lg = dm.out, lep = dq.out;
-          // the cotangent of the smaller term only (both at a tie)
-          float g_m1 = 0.f, g_m0 = 0.f, g_qs = 0.f, g_q0 = 0.f;
-          if (dist || !(lep < lg)) dm.partials(zm1, zm0, LM1, LM0, g_m1, g_m0);
-          if (!(lep > lg)) dq.partials(zqs, zq0, LQs, LQ0, g_qs, g_q0);
+          // (both terms' partials, also the one that the minimum gives no weight: a NaN of either is NaN, and as fast)
+          float g_m1, g_m0, g_qs, g_q0;
+          dm.partials(zm1, zm0, LM1, LM0, g_m1, g_m0);
+          dq.partials(zqs, zq0, LQs, LQ0, g_qs, g_q0);
           const float le1 = fminf(lep, lg);
           const float le2 = kProbFloor + softplus_f(le1 - kProbFloor);
           const float wt = sw_at(esp_at(t));
