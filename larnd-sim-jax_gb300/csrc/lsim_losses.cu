@@ -164,6 +164,10 @@ __global__ void __launch_bounds__(kPairSuper * kPairChunk) k_pair_prepare(PairSo
   if (ok) {
     elo = ehi = src.event[i];
     x = __fadd_rn(src.x[i], __fmul_rn((float)elo, src.offset));
+    if (fabsf(src.x[i]) > kEventOffset / 4) {   // may reach, or swallow, another event's offset: told apart by distance alone
+      elo = -0x7fffffff - 1;
+      ehi = 0x7fffffff;
+    }
     y = src.y[i];
     z = src.z[i];
     w = src.w[i];

@@ -98,3 +98,30 @@ def test_mse_adc_extreme_sigma(cuda, sigma):
     aa, bb = ((w ** 2).sum(), (w * w[::-1]).sum()) if same else (w.sum() ** 2, w.sum() ** 2)
     want = 2 * (float(aa) - float(bb)) / float(w.sum()) ** 2
     assert abs(loss - want) <= 1e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("x0", [3e4, 1.5e5, 1e13, 1e19])
+def test_mse_adc_outside_the_detector(cuda, x0):
+    """Hits so far out that their event's offset does not keep them apart from
+    other events' (a float32 swallows it, or their x makes up for it): every
+    pair counts by its distance."""
+    rng = np.random.default_rng(6)
+    n = 200
+    ev = np.repeat([0, 1], n // 2)
+    def hits(seed):   # noqa: E306
+        h = _hits(rng.uniform(0, 4, n), rng.uniform(0, 4, n), rng.uniform(1, 9, n), ev)
+        h[1][[3, n - 4]] = [x0, x0 if x0 > 1e6 else x0 - 1e5]
+        h[3][n - 4] = h[3][3] + np.float32(0.5)
+        return h
+    a, b = hits(0), hits(1)
+    got = _grads(losses.mse_adc, a, b, lambda_Q=0)
+    X = lambda h: np.stack([(h[1] + h[6].astype(np.float32) * np.float32(1e5)), h[2], h[3]], 1).astype(np.float64)   # noqa: E731
+    w, v = a[0].astype(np.float64), b[0].astype(np.float64)
+    K = lambda p, q: np.exp(-0.5 * ((X(p)[:, None] - X(q)[None]) ** 2).sum(2))   # noqa: E731
+    sw, sv = w.sum(), v.sum()
+    aa, bb, cc = K(a, a) @ w, K(a, b) @ v, K(b, b) @ v
+    want = (w * aa).sum() / sw ** 2 + (v * cc).sum() / sv ** 2 - 2 * (w * bb).sum() / (sw * sv)
+    wq = 2 * aa / sw ** 2 - 2 * (w * aa).sum() / sw ** 3 - 2 * bb / (sw * sv) + 2 * (w * bb).sum() / (sw ** 2 * sv)
+    assert abs(got[0] - want) <= 1e-5 * abs(want)
+    assert np.abs(got[1] - wq).max() <= 1e-5 * np.abs(wq).max()
