@@ -224,7 +224,7 @@ struct ProbArgs {
   float *state;           // [n_pix][H][2][K]: each step's input path charges and log-probabilities
   int32_t *state_top;     // [n_pix][H][K]: each step's selected ticks
   uint32_t *live;         // [n_pix][H][kLiveWords]: ticks whose probability is not 0
-  int32_t *n_run;         // [n_pix]: steps run
+  int32_t *n_run;         // [n_pix]: steps run, kWildRow added for a row that the adjoint takes apart
   float *red;             // [3][n_pix][H]: expected tick and ADC, total probability
 };
 
@@ -236,6 +236,11 @@ constexpr float kProbDead = -104.0f;
 // a path's hit term below this leaves a log-sum-exp above kProbDead as it is:
 // 32 terms of e^-26 next to 1 are below its rounding
 constexpr float kProbFar = kProbDead - 26.0f;
+// The adjoint's partials are finite for arguments up to kWildArgument (the derivative of log_ndtr is exp of a difference
+// that rounds by less than 10 there); rows beyond are marked.
+constexpr float kWildArgument = 1e4f;
+constexpr int32_t kWildRow = 1 << 16;
+static_assert(LSIM_MAX_HITS < kWildRow, "steps and mark");
 // log_diff_ndtr(a, b) <= -1000 sigmoid(-1000 (a - b)): below -1000 sigmoid(-1.4) = -197.8 for a - b < 1.4e-3
 constexpr float kWeakRise = 1.4f, kWeakMost = -190.0f;
 
@@ -325,7 +330,7 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob(ProbArgs a) {
     block_scan_row<kScanSuffixMax>(cr, T, red);
     // rounding of (cm - c) - thr, times z, on both sides of a rise
     float most = fabsf(thr);
-    if (!kDist) {
+    if (!kDist || a.n_run) {
       float m = 0.0f;
       for (int t = tid; t < T; t += kProbThreads) m = fmaxf(m, isfinite(qs[t]) ? fabsf(qs[t]) : INFINITY);
 #pragma unroll
@@ -337,6 +342,7 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob(ProbArgs a) {
       __syncthreads();
     }
     const bool partial = leave_out && isfinite(most);
+    const bool wild = !(most * z < kWildArgument / 2);   // arguments are up to (2 max |q| + |thr|) z
     const float rise = kWeakRise - most * z * (12000.0f / 16777216.0f);
     // esperance values, soft-where weights and the tick classes
     for (int t = tid; t < T - 1; t += kProbThreads) {
@@ -720,7 +726,7 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob(ProbArgs a) {
       __syncthreads();
       continue;
     }
-    if (a.n_run && tid == 0) a.n_run[pix] = h;
+    if (a.n_run && tid == 0) a.n_run[pix] = h | (wild ? kWildRow : 0);
     // the steps that were not run: every probability is exactly 0
     for (int g = h + tid; g < H; g += kProbThreads)
       if (a.lam) {
@@ -854,6 +860,9 @@ constexpr int kPairStride = kProbThreads + 1;   // quantities of one pair in dif
 constexpr int kTickLanes = 4;                   // lanes that share a class's ticks
 static_assert(kProbMaxT <= 65536, "16-bit tick indices");
 
+// Rows whose partials may not be finite (kWildRow) have a launch of their own (kWild): what they need besides costs the
+// others 1.5 % of the adjoint's call.
+template <bool kWild>
 __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va) {
   extern __shared__ __align__(16) float sm[];
   const ProbArgs &a = va.f;
@@ -904,6 +913,7 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
   }
   // the record is only read here: backward passes may share it
   for (int64_t pix = blockIdx.x; pix < a.n_pix; pix += gridDim.x) {
+    if (((a.n_run[pix] & kWildRow) != 0) != kWild) continue;
     const float *w = a.wfs + pix * T;
     for (int t = tid; t < T; t += kProbThreads) qs[t] = w[t] * p.t_sampling;
     __syncthreads();
@@ -941,7 +951,7 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
     const int U = n_cls;
     if (tid == 0) rep[U] = (uint16_t)(T - 1);     // end of the last class
 
-    const int n_run = min(n_exec, a.n_run[pix]);
+    const int n_run = min(n_exec, a.n_run[pix] & (kWildRow - 1));
     if (va.g_lam && n_run < n_exec) {
       // steps left out, every probability of theirs 0: a cotangent that is not finite is NaN on every tick
       bool odd = false;
@@ -1055,6 +1065,13 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
       }
       __syncthreads();
       auto at = [&](int what, int i) -> float & { return pair[what * kPairStride + i]; };
+      // cotangent of the hit log-probability at a tick of probability pr
+      auto cotangent = [&](int tt, float pr) {
+        float gh = 0.f;
+        if (va.g_log_prob) gh = va.g_log_prob[o * (int64_t)(T - 1) + tt];
+        if (va.g_lam) gh += (gl + gt * (float)tt / den + ga * digitize(p, esp_at(tt)) / den) * pr;
+        return gh;
+      };
       const int na = n_act, per_round = kProbThreads / na;   // classes per round of pairs
       const int my = tid / na;                                // this thread's class in a round
       float glp = 0.f, gc = 0.f;                              // cotangents of its path act[tid - my na]
@@ -1075,10 +1092,10 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
           const float LQ0 = log_ndtr_f(zq0), LQs = log_ndtr_f(zqs);
           const LogDiff dq(zqs, zq0, LQs, LQ0, term_m1);
           const float lg = dm.out, lep = dq.out;
-          // (both terms' partials, also the one that the minimum gives no weight: a NaN of either is NaN, and as fast)
-          float g_m1, g_m0, g_qs, g_q0;
-          dm.partials(zm1, zm0, LM1, LM0, g_m1, g_m0);
-          dq.partials(zqs, zq0, LQs, LQ0, g_qs, g_q0);
+          // the partials of the smaller term (both at a tie), and of the other where 0 times it may be NaN
+          float g_m1 = 0.f, g_m0 = 0.f, g_qs = 0.f, g_q0 = 0.f;
+          if (dist || kWild || !(lep < lg)) dm.partials(zm1, zm0, LM1, LM0, g_m1, g_m0);
+          if (kWild || !(lep > lg)) dq.partials(zqs, zq0, LQs, LQ0, g_qs, g_q0);
           const float le1 = fminf(lep, lg);
           const float le2 = kProbFloor + softplus_f(le1 - kProbFloor);
           const float wt = sw_at(esp_at(t));
@@ -1142,6 +1159,18 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
           const int e = i / kTickLanes;
           const bool mine = e < n_round;
           float Hs = 0.f, Ds = 0.f, inv = 0.f, inv_d = 0.f;
+          // a class without a cotangent takes no part, which shows only where its sums are not finite
+          bool takes_part = true;
+          if (kWild) {
+            bool any = false;
+            if (mine) {
+              const int u = list[e0 + e];
+              const float pr = expf(logf(at(kPairSums, e * na)) + at(kPairMax, e * na));
+              for (int tt = rep[u] + i % kTickLanes; tt < rep[u + 1]; tt += kTickLanes)
+                any |= cotangent(tt, pr) != 0.f || Gd[tt] != 0.f;
+            }
+            takes_part = (__ballot_sync(0xffffffffu, any) >> (lane & ~(kTickLanes - 1))) & ((1u << kTickLanes) - 1u);
+          }
           if (mine) {
             const int u = list[e0 + e], f = e * na;
             const bool with_d = tmp[u] != 0.f;
@@ -1149,14 +1178,12 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
             inv = 1.0f / S;
             inv_d = with_d ? 1.0f / at(kPairDistSums, f) : 0.f;
             for (int tt = rep[u] + i % kTickLanes; tt < rep[u + 1]; tt += kTickLanes) {
-              float gh = 0.f, add_e = 0.f;
-              const float gd = Gd[tt];
-              if (va.g_log_prob) gh = va.g_log_prob[o * (int64_t)(T - 1) + tt];
-              if (va.g_lam) {
-                const float et = esp_at(tt);
-                gh += (gl + gt * (float)tt / den + ga * digitize(p, et) / den) * pr;
-                add_e = digitize_vjp(p, et, ga * pr / den);
+              const float add_e = va.g_lam ? digitize_vjp(p, esp_at(tt), ga * pr / den) : 0.f;
+              if (!takes_part) {
+                Aesp[tt] += add_e;
+                continue;
               }
+              const float gh = cotangent(tt, pr), gd = Gd[tt];
               Hs += gh;
               Ds += gd;
               const float n = gh * inv, nd = gd * inv_d;
@@ -1178,20 +1205,21 @@ __global__ void __launch_bounds__(kProbThreads, 2) k_fee_prob_vjp(ProbVjpArgs va
             Ds += __shfl_xor_sync(0xffffffffu, Ds, s2);
           }
           if (mine && i % kTickLanes == 0) {
-            at(kPairMax, e * na) = Hs * inv;
+            at(kPairMax, e * na) = Hs != 0.f ? Hs * inv : 0.f;
             at(kPairDistSums, e * na) = Ds * inv_d;
           }
         }
         __syncthreads();
         // ---- the pair's path (the next round writes these two values only after its first barrier)
         if (on) {
-          const float n = at(kPairMax, my * na);
-          glp += wh * n;
-          gc -= gh_c * n;
-          if (dist) {
-            const float nd = at(kPairDistSums, my * na);
-            glp += wd * nd;
-            gc -= gd_c * nd;
+          const float n = at(kPairMax, my * na), nd = dist ? at(kPairDistSums, my * na) : 0.f;
+          if (!kWild || n != 0.f || nd != 0.f) {
+            glp += wh * n;
+            gc -= gh_c * n;
+            if (dist) {
+              glp += wd * nd;
+              gc -= gd_c * nd;
+            }
           }
         }
       }
@@ -1376,11 +1404,23 @@ static int run_fee_prob_impl(const LsimParams &p, const float *wfs, int64_t n_pi
   return cudaGetLastError() == cudaSuccess ? LSIM_OK : LSIM_ERR_CUDA;
 }
 
+template <bool kWild>
+static int launch_vjp(const ProbVjpArgs &va, cudaStream_t st) {
+  const size_t smem = sizeof(float) * (kVjpArrays * kProbMaxT + kPairValues * kPairStride) +
+                      sizeof(uint16_t) * kVjpShorts * kProbMaxT;
+  if (cudaFuncSetAttribute(k_fee_prob_vjp<kWild>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+      cudaSuccess)
+    return LSIM_ERR_CUDA;
+  constexpr int64_t cap = 1 << 30;
+  k_fee_prob_vjp<kWild><<<(unsigned)(va.f.n_pix < cap ? va.f.n_pix : cap), kProbThreads, smem, st>>>(va);
+  return cudaGetLastError() == cudaSuccess ? LSIM_OK : LSIM_ERR_CUDA;
+}
+
 // The reverse pass on a record.
 int run_fee_prob_vjp_recorded(const LsimParams &p, const float *wfs, int64_t n_pix, int32_t n_t, int32_t n_paths,
                               const void *record, const float *g_log_prob, const float *g_charge, const float *g_e_tick,
                               const float *g_e_adc, const float *g_lam, float *g_wfs, cudaStream_t st) {
-  const int rc = check_prob(p, n_t, n_paths);
+  int rc = check_prob(p, n_t, n_paths);
   if (rc != LSIM_OK || n_pix == 0) return rc;
   ProbRecord r;
   record_layout(n_pix, p.max_adc_values, n_paths, &r, const_cast<char *>(static_cast<const char *>(record)));
@@ -1399,17 +1439,12 @@ int run_fee_prob_vjp_recorded(const LsimParams &p, const float *wfs, int64_t n_p
   va.g_e_adc = g_e_adc;
   va.g_lam = g_lam;
   va.g_wfs = g_wfs;
-  const size_t smem = sizeof(float) * (kVjpArrays * kProbMaxT + kPairValues * kPairStride) +
-                      sizeof(uint16_t) * kVjpShorts * kProbMaxT;
-  if (cudaFuncSetAttribute(k_fee_prob_vjp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return LSIM_ERR_CUDA;
   // a block per pixel: pixels differ several times in cost, and blocks start as
   // others end (the record is only read, so it has no place for a counter).
   // 1500 rows, with a warp per class: 5.6 ms with the rows dealt in turn to the
   // resident blocks, 4.8 ms so
-  constexpr int64_t cap = 1 << 30;
-  k_fee_prob_vjp<<<(unsigned)(n_pix < cap ? n_pix : cap), kProbThreads, smem, st>>>(va);
-  return cudaGetLastError() == cudaSuccess ? LSIM_OK : LSIM_ERR_CUDA;
+  rc = launch_vjp<false>(va, st);
+  return rc != LSIM_OK ? rc : launch_vjp<true>(va, st);
 }
 
 size_t fee_prob_vjp_workspace_bytes(int64_t n_pix, int32_t max_adc_values, int32_t n_paths) {

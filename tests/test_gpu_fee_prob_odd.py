@@ -75,3 +75,18 @@ def test_hit_without_cotangent(cuda, hit):
     assert lam[0, 0] == 1 and 1e-8 < lam[0, 1] < 2e-8
     lam[0, hit].backward()
     assert bool(torch.isnan(w.grad).all()) if hit else bool(torch.isfinite(w.grad).all())
+
+
+def test_partials_without_weight(cuda):
+    """A row that falls and rises by 1e31: where the minimum of a hit's two
+    terms gives the one with a NaN partial no weight, 0 times it is NaN."""
+    import torch
+    w = np.random.default_rng(3).normal(300, 2000, (4, 65)).astype(np.float32)
+    w[1, 1], w[1, 26] = -1e31, 1e31
+    params = consts.Params(fee_paths_scaling=20, RESET_NOISE_CHARGE=50, DISCRIMINATION_THRESHOLD=-200)
+    x = torch.from_numpy(w).cuda().requires_grad_(True)
+    out = sim.average_hit_values(params, x)
+    assert all(bool(torch.isfinite(o).all()) for o in out)
+    torch.autograd.backward(out, [torch.ones_like(o) for o in out])
+    odd = torch.isnan(x.grad).any(1).tolist()
+    assert odd == [False, True, False, False]
