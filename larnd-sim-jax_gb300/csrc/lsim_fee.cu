@@ -366,9 +366,9 @@ __device__ __forceinline__ float quad(const float c[6], float x, float y) {
 // at the default 51 ticks, dealt over the lanes without idle ones) and
 // writes the samples per segment; k_param_pixels adds them in slot order.
 // Bound by the special functions' instructions in the first, by the rows
-// written in the second.  param_wfs of 32 events (0.3M segments): 2.07 -> 0.91
+// written in the second.  param_wfs of 32 events (0.3M segments): 2.07 -> 0.80
 // ms; with the adjoint split likewise (below), a gradient step of 16 events:
-// 4.79 -> 3.04 ms.
+// 5.33 -> 2.68 ms (both with the smaller launches around them).
 constexpr int kParWarps = 4;
 constexpr int kParTicks = 64;               // most ticks of a window (checked by the host)
 constexpr int kParEdges = 2 * kParTicks;

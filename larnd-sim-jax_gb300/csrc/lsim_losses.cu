@@ -94,7 +94,9 @@ constexpr int kPairChunk = 32;    // column hits per chunk
 constexpr int kPairSuper = 32;    // chunks per entry of the upper event-range list
 constexpr int kPairWarps = 4;     // warps per block
 constexpr int kPairMaxSlices = 16;
-constexpr int kPairWantWarps = 4864;   // 152 SMs x 32 warps: below this the columns are sliced
+// below this the columns are sliced: 152 SMs x 32 warps, a constant so that the
+// slices, hence the bits and the workspace, follow the counts of hits alone
+constexpr int kPairWantWarps = 4864;
 constexpr float kCutMse = 64.f, kCutNll = 100.f;
 constexpr float kCutZero = 150.f;      // 2^-150 and below round to 0
 constexpr float kLeftOut = 67108864.f; // 2^26: a quarter of a float32's last place
@@ -541,8 +543,9 @@ struct MseAdcTotals {
   float loss, mmd, charge;
 };
 
-// Block sums of up to kRedMax doubles per thread: warp sums, then thread 0
-// adds the warps' in order into out[q].
+// Block sums of up to kRedMax doubles per thread: warp sums, then a thread per
+// sum adds the warps' in order into out[q].  (At most kRedBlocks blocks, a
+// constant for the same reason as the slices.)
 constexpr int kRedBlocks = 304, kRedThreads = 256, kRedMax = 5;
 
 template <int N>
